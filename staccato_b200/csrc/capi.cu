@@ -360,25 +360,28 @@ namespace {
 
 // A validated, classified and ordered sweep: the host image of the device metadata
 // (descriptors, cost-ordered work lists, fallback list, zeroed counters) plus launch shapes.
-// Storage classes of a plan: 0 FP64 shared-memory kernel, 1 global kernel (FP64, or the
-// CUDA-core mixed kernel), 2 large-order FP64 kernel, 3 tensor-core mixed kernel.
-constexpr int NCLS = 4;
+// Storage classes of a plan: 0 FP64 orders whose matrix fits shared memory (routed to the row
+// kernel), 1 global kernel (FP64 above n = 512, or the CUDA-core mixed kernel), 2 large-order FP64
+// kernel, 3 tensor-core mixed kernel, 4..7 the FP64 row kernel (sweep_lu64.cu) with 64, 128, 256
+// and 512 threads a system.
+constexpr int NCLS = 8;
+constexpr int CLS_ROW = 4, N_ROW = 4;
 
 struct SweepPlan {
     bool mixed = false;
     srom_sweep_opts o{};
     std::vector<char> meta;
-    size_t off_items[NCLS] = {0, 0, 0, 0};
+    size_t off_items[NCLS] = {};
     size_t off_fb = 0, off_ctr = 0;
-    long long n_items[NCLS] = {0, 0, 0, 0};
-    double flops[NCLS] = {0.0, 0.0, 0.0, 0.0};
-    size_t smem_max = 0;
+    long long n_items[NCLS] = {};
+    double flops[NCLS] = {};
     int g_nmax = 0, g_rmax = 0;    // class 1: the global kernels' largest order and RHS count
     int b_nmax = 0, b_rmax = 0;    // class 2: the large-order FP64 kernel's
     int t_nmax = 0, t_rmax = 0;    // class 3: the tensor-core kernel's
     int f_nmax = 0, f_rmax = 0;    // the FP64 re-solve of non-converged mixed systems (classes 1, 3)
-    long long grid0 = 0, grid1 = 0, grid2 = 0, grid3 = 0;
-    int64_t slot_bytes = 0, slot2_bytes = 0, slot3_bytes = 0, slotf_bytes = 0;
+    int r_nmax[N_ROW] = {}, r_rmax[N_ROW] = {};  // classes 4..7
+    long long grid1 = 0, grid2 = 0, grid3 = 0, gridr[N_ROW] = {}, gridf = 0;
+    int64_t slot_bytes = 0, slot2_bytes = 0, slot3_bytes = 0, slotf_bytes = 0, slotr_bytes[N_ROW] = {};
     bool need_scratch = false;
     std::vector<srom::BackProj> backproj;  // ROMs whose solutions are projected onto outputs
     // ROMs without a mass matrix.  Their descriptors point M at a zero matrix instead: for any
@@ -410,6 +413,15 @@ int fp64_class(const srom_handle *h, int n, int r) {
     return 0;
 }
 
+// Thread counts of the FP64 row kernel's classes: the smallest with a thread a row (wide: the next
+// one up).
+constexpr int row_threads(int q) { return 64 << q; }
+int row_class(int n, bool wide) {
+    int q = 0;
+    while (row_threads(q) < n) ++q;
+    return std::min(q + (wide ? 1 : 0), N_ROW - 1);
+}
+
 // Mixed-form class: a system the FP64 shared-memory kernel holds two or more at a time per SM
 // is solved there outright.  At those orders (n <= ~84 for r <= 4) one FP64 factorisation in
 // shared memory is faster than complex-FP32 factors in the global kernel plus refinement
@@ -423,7 +435,7 @@ int mixed_class(const srom_handle *h, int n, int r, int flags) {
     if (fp64_class(h, n, r) != 0) return 1;
     auto it = h->tune_mixed.find(((long long)n << 16) | r);  // srom_tune's measurement, if any
     if (it != h->tune_mixed.end()) return it->second;
-    return srom::fp64_smem_blocks_per_sm(srom::fp64_smem_bytes(n, r)) >= 2 ? 0 : 1;
+    return 2 * (srom::fp64_smem_bytes(n, r) + 1024) <= (size_t)h->max_smem_optin + 1024 ? 0 : 1;
 }
 
 // SROM_MIXED_AUTO: the tensor-core kernel from this order up (without a measurement).  On the
@@ -508,24 +520,11 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
             for (int i = 0; i < n_roms; ++i)
                 if (cls[i] == 3) cls[i] = 1;
     }
-    for (int i = 0; i < n_roms; ++i) {
-        const srom_rom_desc &d = roms[i];
-        if (cls[i] < 0) continue;
-        if (cls[i] == 0) {
-            P.smem_max = std::max(P.smem_max, srom::fp64_smem_bytes(d.n, d.r));
-        } else if (cls[i] == 1) {
-            P.g_nmax = std::max(P.g_nmax, d.n);
-            P.g_rmax = std::max(P.g_rmax, d.r);
-        } else if (cls[i] == 2) {
-            P.b_nmax = std::max(P.b_nmax, d.n);
-            P.b_rmax = std::max(P.b_rmax, d.r);
-        } else {
-            P.t_nmax = std::max(P.t_nmax, d.n);
-            P.t_rmax = std::max(P.t_rmax, d.r);
+    for (int i = 0; i < n_roms; ++i)
+        if (cls[i] == 2) {
+            P.b_nmax = std::max(P.b_nmax, roms[i].n);
+            P.b_rmax = std::max(P.b_rmax, roms[i].r);
         }
-        P.n_items[cls[i]] += d.F;
-        P.flops[cls[i]] += lu_flops(d.n, d.r) * d.F;
-    }
     if (P.b_nmax > srom::BIG_MAX_N)
         return set_err(h, SROM_ERR_UNSUPPORTED, "n=%d exceeds the largest supported order %d", P.b_nmax,
                        srom::BIG_MAX_N);
@@ -533,17 +532,36 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
         return set_err(h, SROM_ERR_UNSUPPORTED,
                        "n=%d with r=%d: the right-hand sides (n*r*16 bytes) exceed shared memory", P.b_nmax,
                        P.b_rmax);
-    if (P.n_items[0] + P.n_items[1] + P.n_items[2] + P.n_items[3] > INT32_MAX)
-        return set_err(h, SROM_ERR_UNSUPPORTED, "too many systems");
-    if (P.n_items[0] > 0) {
-        const int bps = srom::fp64_smem_blocks_per_sm(P.smem_max);
-        if (bps <= 0) return set_err(h, SROM_ERR_UNSUPPORTED, "smem kernel cannot be resident (%zu B)", P.smem_max);
-        P.grid0 = std::min<long long>(P.n_items[0], (long long)bps * h->sm_count);
+    // FP64 systems of orders up to 512 run on the row kernel; a measured "global" choice of
+    // srom_tune gives such a system the next larger thread count
+    P.b_nmax = P.b_rmax = 0;
+    for (int i = 0; i < n_roms; ++i) {
+        const srom_rom_desc &d = roms[i];
+        if (cls[i] < 0) continue;
+        if (d.n <= srom::LU64_MAX_N && (cls[i] == 0 || cls[i] == 2 || (cls[i] == 1 && !mixed)))
+            cls[i] = CLS_ROW + row_class(d.n, cls[i] == 1 && srom::fp64_smem_bytes(d.n, d.r) <= smem_cap);
+        const int c = cls[i];
+        int *nm = c == 1 ? &P.g_nmax : c == 2 ? &P.b_nmax : c == 3 ? &P.t_nmax : &P.r_nmax[c - CLS_ROW];
+        int *rm = c == 1 ? &P.g_rmax : c == 2 ? &P.b_rmax : c == 3 ? &P.t_rmax : &P.r_rmax[c - CLS_ROW];
+        *nm = std::max(*nm, d.n);
+        *rm = std::max(*rm, d.r);
+        P.n_items[c] += d.F;
+        P.flops[c] += lu_flops(d.n, d.r) * d.F;
+    }
+    long long all_items = 0;
+    for (int c = 0; c < NCLS; ++c) all_items += P.n_items[c];
+    if (all_items > INT32_MAX) return set_err(h, SROM_ERR_UNSUPPORTED, "too many systems");
+    for (int q = 0; q < N_ROW; ++q) {
+        if (P.n_items[CLS_ROW + q] == 0) continue;
+        P.gridr[q] = std::min<long long>(P.n_items[CLS_ROW + q],
+                                         (long long)srom::lu64_blocks_per_sm(row_threads(q), P.r_nmax[q]) * h->sm_count);
+        P.slotr_bytes[q] = srom::lu64_slot_bytes(P.r_nmax[q], P.r_rmax[q]);
+        P.need_scratch = true;
     }
     if (P.n_items[1] > 0) {
         P.grid1 = std::min<long long>(P.n_items[1], h->sm_count);
         P.slot_bytes = (int64_t)P.g_nmax * P.g_nmax * (int64_t)sizeof(double2);
-        P.need_scratch = mixed;
+        P.need_scratch = P.need_scratch || mixed;
         for (int i = 0; i < n_roms; ++i)
             if (cls[i] == 1 && !roms[i].LU) P.need_scratch = true;
     }
@@ -553,12 +571,16 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
         P.need_scratch = true;
     }
     if (mixed && (o.flags & SROM_FLAG_FALLBACK_FP64) && P.n_items[1] + P.n_items[3] > 0) {
-        // the FP64 re-solve covers the systems of both mixed kernels, one CTA per SM
+        // the FP64 re-solve covers the systems of both mixed kernels
         P.f_nmax = std::max(P.g_nmax, P.t_nmax);
         P.f_rmax = std::max(P.g_rmax, P.t_rmax);
-        P.slotf_bytes = srom::global_panel_fits(P.f_nmax, P.f_rmax, h->max_smem_optin)
-                            ? (int64_t)P.f_nmax * P.f_nmax * (int64_t)sizeof(double2)
-                            : srom::big_slot_bytes(P.f_nmax);
+        P.gridf = std::max(P.grid1, P.grid3);
+        if (P.f_nmax <= srom::LU64_MAX_N)
+            P.slotf_bytes = srom::lu64_slot_bytes(P.f_nmax, P.f_rmax);
+        else if (srom::global_panel_fits(P.f_nmax, P.f_rmax, h->max_smem_optin))
+            P.slotf_bytes = (int64_t)P.f_nmax * P.f_nmax * (int64_t)sizeof(double2);
+        else
+            P.slotf_bytes = srom::big_slot_bytes(P.f_nmax);
     }
     if (P.n_items[2] > 0) {
         // one system per CTA: matrix (or the caller's LU buffer) and the panel in the CTA's slot;
@@ -581,7 +603,7 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
     if (n_roms) memcpy(hm, dev.data(), sizeof(RomDev) * n_roms);
     Item *its[NCLS];
     for (int c = 0; c < NCLS; ++c) its[c] = reinterpret_cast<Item *>(hm + P.off_items[c]);
-    long long k[NCLS] = {0, 0, 0, 0};
+    long long k[NCLS] = {};
     for (int oi = 0; oi < n_roms; ++oi) {
         const int i = order[oi];
         if (cls[i] < 0) continue;
@@ -595,25 +617,38 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
 size_t plan_scratch_bytes(const SweepPlan &P) {
     size_t b = std::max<size_t>((size_t)P.slot_bytes * P.grid1, (size_t)P.slot2_bytes * P.grid2);
     b = std::max<size_t>(b, (size_t)P.slot3_bytes * P.grid3);
-    return std::max<size_t>(b, (size_t)P.slotf_bytes * std::max(P.grid1, P.grid3));
+    for (int q = 0; q < N_ROW; ++q) b = std::max<size_t>(b, (size_t)P.slotr_bytes[q] * P.gridr[q]);
+    return std::max<size_t>(b, (size_t)P.slotf_bytes * P.gridf);
 }
 
 // Counters live at off_ctr and must be zero when the launches start (the metadata copy zeroes
-// them, or zero_counters does): 0 smem kernel, 1 global kernel, 2 fallback count, 3 fallback
-// work, 4 tensor-core error word, 5 large-order kernel, 6 tensor-core kernel.
+// them, or zero_counters does): 1 global kernel, 2 fallback count, 3 fallback work, 4 tensor-core
+// error word, 5 large-order kernel, 6 tensor-core kernel, 8..11 row kernel.
 int enqueue_plan(srom_handle *h, const SweepPlan &P, char *dm, void *scratch, cudaStream_t st, bool zero_counters,
                  bool profile) {
     const RomDev *d_roms = reinterpret_cast<const RomDev *>(dm);
     auto items = [&](int c) { return reinterpret_cast<const Item *>(dm + P.off_items[c]); };
     int *d_ctr = reinterpret_cast<int *>(dm + P.off_ctr);
-    if (zero_counters) SROM_CUDA(h, cudaMemsetAsync(d_ctr, 0, 8 * sizeof(int), st));
+    if (zero_counters) SROM_CUDA(h, cudaMemsetAsync(d_ctr, 0, 16 * sizeof(int), st));
     const bool prof_prev = h->prof;
     if (!profile) h->prof = false;
     int rc = SROM_OK;
-    if (P.n_items[0] > 0) {
-        ProfScope ps(h, "fp64_smem", P.n_items[0], P.flops[0], 0.0);
-        cudaError_t e = srom::launch_fp64_smem(d_roms, items(0), (int)P.n_items[0], d_ctr, P.smem_max, (int)P.grid0, st);
-        if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "fp64 smem launch: %s", cudaGetErrorString(e));
+    // the largest orders first, so that the small systems fill the last waves
+    for (int q = N_ROW - 1; q >= 0 && rc == SROM_OK; --q) {
+        const int c = CLS_ROW + q;
+        if (P.n_items[c] == 0) continue;
+        srom::GlobalArgs a{};
+        a.roms = d_roms;
+        a.items = items(c);
+        a.n_items = (int)P.n_items[c];
+        a.counter = d_ctr + 8 + q;
+        a.scratch = static_cast<unsigned char *>(scratch);
+        a.slot_bytes = P.slotr_bytes[q];
+        a.n_max = P.r_nmax[q];
+        a.r_max = P.r_rmax[q];
+        ProfScope ps(h, q < 2 ? "fp64_smem" : "fp64_global", P.n_items[c], P.flops[c], 0.0);
+        cudaError_t e = srom::launch_lu64(row_threads(q), a, (int)P.gridr[q], st);
+        if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "fp64 row launch: %s", cudaGetErrorString(e));
     }
     Item *fb_items = nullptr;
     int *fb_count = nullptr;
@@ -664,9 +699,10 @@ int enqueue_plan(srom_handle *h, const SweepPlan &P, char *dm, void *scratch, cu
         b.n_max = P.f_nmax;
         b.r_max = P.f_rmax;
         b.steps_value = -1;
-        const int grid = (int)std::max(P.grid1, P.grid3);
+        const int grid = (int)P.gridf;
         ProfScope ps(h, "fp64_fallback", 0, 0.0, 0.0);
-        cudaError_t e = srom::global_panel_fits(P.f_nmax, P.f_rmax, h->max_smem_optin)
+        cudaError_t e = P.f_nmax <= srom::LU64_MAX_N ? srom::launch_lu64(row_threads(row_class(P.f_nmax, false)), b, grid, st)
+                        : srom::global_panel_fits(P.f_nmax, P.f_rmax, h->max_smem_optin)
                             ? srom::launch_global(false, b, grid, st)
                             : srom::launch_global_big(b, grid, st);
         if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "fallback launch: %s", cudaGetErrorString(e));

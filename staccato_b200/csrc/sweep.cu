@@ -3,17 +3,14 @@
 // One CTA owns one (ROM, frequency) system at a time and pulls the next one from a work
 // counter (persistent launch; the host orders the work list largest systems first).
 //
-// Storage classes
-//   smem   : whole n x n FP64 matrix and right-hand sides in shared memory (n up to ~112);
-//            unblocked right-looking LU, one warp searches each pivot.
-//   global : matrix in a per-CTA scratch slot (L2-resident while in flight); blocked
-//            right-looking LU.  The NB-column panel is staged in shared memory and factored
-//            by all warps with one CTA barrier per column: row interchanges are tracked as a
-//            logical permutation, so no row is physically moved while the column is being
-//            searched.  After the panel, every warp independently processes its own groups
-//            of CW trailing columns: apply the panel's interchanges, solve the unit-lower
-//            triangle for the U rows (warp shuffles), and update the remaining rows with
-//            register-tiled complex FMAs.  No CTA barrier separates the column groups.
+// Storage: the matrix lives in a per-CTA scratch slot (L2-resident while in flight); blocked
+// right-looking LU.  The NB-column panel is staged in shared memory and factored by all warps with
+// one CTA barrier per column: row interchanges are tracked as a logical permutation, so no row is
+// physically moved while the column is being searched.  After the panel, every warp independently
+// processes its own groups of CW trailing columns: apply the panel's interchanges, solve the
+// unit-lower triangle for the U rows (warp shuffles), and update the remaining rows with
+// register-tiled complex FMAs.  No CTA barrier separates the column groups.  FP64 systems of orders up
+// to 512 run on the row kernel of sweep_lu64.cu instead.
 //
 // Precision forms
 //   FP64  (double2): reproduces LAPACK zgetrf/zgetrs as restated in the oracle bit for bit:
@@ -40,80 +37,6 @@
 #include "sweep_common.cuh"
 
 namespace srom {
-
-
-// ====================================================================================
-// smem class (FP64)
-// ====================================================================================
-__device__ __forceinline__ void panel_factor_smem(double2 *P, int ldp, int m, int ncols, int *ipiv, int *s_info,
-                                  double2 *Bs, int ldbs, int nrhs, int *s_bc) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int jj = 0; jj < ncols; ++jj) {
-        if (warp == 0) {
-            double best = -1.0;
-            int bi = INT_MAX;
-            for (int i = jj + lane; i < m; i += 32) {
-                double v = cabs1(P[i + (int64_t)jj * ldp]);
-                if (v > best) {
-                    best = v;
-                    bi = i;
-                }
-            }
-#pragma unroll
-            for (int off = 16; off; off >>= 1) {
-                double ob = __shfl_xor_sync(FULL_MASK, best, off);
-                int oi = __shfl_xor_sync(FULL_MASK, bi, off);
-                if (ob > best || (ob == best && oi < bi)) {
-                    best = ob;
-                    bi = oi;
-                }
-            }
-            // IZAMAX starts from the first entry: a NaN there is returned as the pivot.
-            double first = cabs1(P[jj + (int64_t)jj * ldp]);
-            if (bi == INT_MAX || first != first) bi = jj;
-            double2 piv = P[bi + (int64_t)jj * ldp];
-            bool nz = (piv.x != 0.0 || piv.y != 0.0);
-            if (nz) {
-                if (bi != jj) {
-                    if (lane == 0) {
-                        P[bi + (int64_t)jj * ldp] = P[jj + (int64_t)jj * ldp];
-                        P[jj + (int64_t)jj * ldp] = piv;
-                    }
-                    if (Bs)
-                        for (int c = lane; c < nrhs; c += 32)
-                            swap2(Bs[jj + (int64_t)c * ldbs], Bs[bi + (int64_t)c * ldbs]);
-                }
-                __syncwarp();
-                double2 inv = crecip(piv);
-                for (int i = jj + 1 + lane; i < m; i += 32)
-                    P[i + (int64_t)jj * ldp] = cmul(P[i + (int64_t)jj * ldp], inv);
-            } else if (lane == 0 && *s_info == 0) {
-                *s_info = jj + 1;
-            }
-            if (lane == 0) {
-                s_bc[0] = bi;
-                s_bc[1] = nz ? 1 : 0;
-                ipiv[jj] = bi + 1;
-            }
-        }
-        __syncthreads();
-        const int p = s_bc[0];
-        const bool doswap = s_bc[1] && p != jj;
-        if (doswap)
-            for (int c = tid; c < jj; c += NT) swap2(P[jj + (int64_t)c * ldp], P[p + (int64_t)c * ldp]);
-        for (int c = jj + 1 + warp; c < ncols; c += NW) {
-            double2 *col = P + (int64_t)c * ldp;
-            if (doswap) {
-                if (lane == 0) swap2(col[jj], col[p]);
-                __syncwarp();
-            }
-            const double2 u = col[jj];
-            const double2 *lcol = P + (int64_t)jj * ldp;
-            for (int i = jj + 1 + lane; i < m; i += 32) col[i] = csubmul(col[i], lcol[i], u);
-        }
-        __syncthreads();
-    }
-}
 
 
 // One row of the blocked substitution: b[i, c] -= sum_j A[i, j] b[j, c] over the block's
@@ -365,43 +288,6 @@ __device__ void lu_solve_strips(const T *A, int64_t lda, int n, T *B, int ldb, i
     }
 }
 
-
-__global__ void __launch_bounds__(NT) sweep_fp64_smem_kernel(const RomDev *__restrict__ roms,
-                                                              const Item *__restrict__ items,
-                                                              int n_items, int *counter) {
-    extern __shared__ double2 smem[];
-    __shared__ int s_item, s_info, s_bc[2];
-    for (;;) {
-        const int it = next_item(counter, &s_item);
-        if (it >= n_items) break;
-        const Item w = items[it];
-        const RomDev R = roms[w.rom];
-        const int n = R.n;
-        const int lda = n | 1;
-        double2 *A = smem;
-        double2 *B = A + (int64_t)n * lda;
-        int *ipiv = reinterpret_cast<int *>(B + (int64_t)n * R.r);
-        assemble_into<double2>(A, lda, R, R.omega[w.f], w.f);
-        load_rhs(B, n, R);
-        if (threadIdx.x == 0) s_info = 0;
-        __syncthreads();
-        panel_factor_smem(A, lda, n, n, ipiv, &s_info, B, n, R.r, s_bc);
-        lu_solve<double2>(A, lda, n, B, n, R.r, nullptr);
-        store_solution(B, n, R, w.f);
-        if (R.LU) {
-            double2 *LU = R.LU + (int64_t)w.f * n * n;
-            for (int j = threadIdx.x >> 5; j < n; j += NW)
-                for (int i = threadIdx.x & 31; i < n; i += 32) LU[i + (int64_t)j * n] = A[i + j * lda];
-            for (int j = threadIdx.x; j < n; j += NT) R.ipiv[(int64_t)w.f * n + j] = ipiv[j];
-        }
-        if (threadIdx.x == 0) {
-            if (R.info) R.info[w.f] = s_info;
-            if (R.steps) R.steps[w.f] = 0;
-            if (R.berr) R.berr[w.f] = 0.0;
-        }
-        __syncthreads();
-    }
-}
 
 // ====================================================================================
 // global class
@@ -745,23 +631,6 @@ size_t fp64_global_smem_bytes(int n_max, int r_max) { return global_smem_bytes(n
 
 int global_rpt(int n_max) { return (n_max + NT - 1) / NT; }
 
-cudaError_t launch_fp64_smem(const RomDev *roms, const Item *items, int n_items, int *counter,
-                             size_t smem, int grid, cudaStream_t st) {
-    auto k = sweep_fp64_smem_kernel;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k<<<grid, NT, smem, st>>>(roms, items, n_items, counter);
-    return cudaGetLastError();
-}
-
-int fp64_smem_blocks_per_sm(size_t smem) {
-    int b = 0;
-    auto k = sweep_fp64_smem_kernel;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, NT, smem) != cudaSuccess) return 0;
-    return b;
-}
-
 // The mixed kernel takes all the shared memory a CTA may have (one CTA per SM either way, by
 // registers): what lies beyond its fixed regions deepens the correction solves' staging ring.
 template <bool MIXED, int RPT, bool BIG = false>
@@ -799,9 +668,7 @@ cudaError_t launch_global(bool mixed, const GlobalArgs &a0, int grid, cudaStream
         if (rpt == 2) return launch_global_t<true, 2>(a, grid, st);
         if (rpt == 3) return launch_global_t<true, 3>(a, grid, st);
     } else {
-        if (rpt <= 1) return launch_global_t<false, 1>(a, grid, st);
-        if (rpt == 2) return launch_global_t<false, 2>(a, grid, st);
-        if (rpt == 3) return launch_global_t<false, 3>(a, grid, st);
+        if (rpt <= 3) return launch_global_t<false, 3>(a, grid, st);  // n > LU64_MAX_N
     }
     return cudaErrorInvalidValue;
 }
@@ -816,21 +683,6 @@ cudaError_t launch_global_big(const GlobalArgs &a0, int grid, cudaStream_t st) {
     if (rpt <= 6) return launch_global_t<false, 6, true>(a, grid, st);
     if (rpt <= BIG_RPT) return launch_global_t<false, BIG_RPT, true>(a, grid, st);
     return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_fp64_global(const RomDev *roms, const Item *items, int n_items, int *counter,
-                               double2 *scratch, int64_t slot_elems, int n_max, int r_max, int grid,
-                               cudaStream_t st) {
-    GlobalArgs a{};
-    a.roms = roms;
-    a.items = items;
-    a.n_items = n_items;
-    a.counter = counter;
-    a.scratch = reinterpret_cast<unsigned char *>(scratch);
-    a.slot_bytes = slot_elems * (int64_t)sizeof(double2);
-    a.n_max = n_max;
-    a.r_max = r_max;
-    return launch_global(false, a, grid, st);
 }
 
 }  // namespace srom

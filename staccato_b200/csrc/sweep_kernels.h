@@ -16,11 +16,10 @@ struct Item;
 inline bool misaligned(const void *p, size_t a) { return p && (reinterpret_cast<uintptr_t>(p) % a) != 0; }
 
 // ---- FP64 (bit-identical to the restated zgetrf/zgetrs) ----
+// bytes of a whole n x n system with its right-hand sides and pivots: the small orders are those
+// whose system fits a CTA's shared memory
 size_t fp64_smem_bytes(int n, int r);
 size_t fp64_global_smem_bytes(int n_max, int r_max);
-int fp64_smem_blocks_per_sm(size_t smem);
-cudaError_t launch_fp64_smem(const RomDev *roms, const Item *items, int n_items, int *counter,
-                             size_t smem, int grid, cudaStream_t st);
 // dynamic shared memory of the global kernels; big: the large-order FP64 instances
 size_t global_smem_bytes(int n_max, int r_max, bool big = false);
 // the shared-memory-panel instances (launch_global) can run (n_max, r_max)
@@ -58,9 +57,13 @@ cudaError_t launch_global(bool mixed, const GlobalArgs &a, int grid, cudaStream_
 // FP64 sweep of orders up to BIG_MAX_N with the panel in global scratch (slot_bytes >=
 // big_slot_bytes(n_max)); 3, 6 or 10 rows per thread by n_max
 cudaError_t launch_global_big(const GlobalArgs &a, int grid, cudaStream_t st);
-cudaError_t launch_fp64_global(const RomDev *roms, const Item *items, int n_items, int *counter,
-                               double2 *scratch, int64_t slot_elems, int n_max, int r_max,
-                               int grid, cudaStream_t st);
+
+// ---- FP64, orders up to LU64_MAX_N (sweep_lu64.cu): one thread a row, Schur updates on the FP64
+// tensor cores; threads = 64, 128, 256 or 512, at least n_max ----
+constexpr int LU64_MAX_N = 512;
+int lu64_blocks_per_sm(int threads, int n_max);
+int64_t lu64_slot_bytes(int n_max, int r_max);  // global scratch per CTA
+cudaError_t launch_lu64(int threads, const GlobalArgs &a, int grid, cudaStream_t st);
 
 // ---- tensor-core mixed form (sweep_tc.cu): complex-FP32 LU whose Schur updates run as
 // tcgen05 MMAs on three-piece bf16 splits, FP64 refinement as in the global kernel ----
