@@ -34,6 +34,10 @@ struct AdjointArgs {
 };
 
 size_t adjoint_smem_bytes(int n, int r, int n_terms);
-cudaError_t launch_adjoint(const AdjointArgs &a, int n, int r, int F, int grid, double *dJdp, cudaStream_t st);
+// Device workspace of launch_adjoint (own_lambda: the caller gives no lambda array).
+size_t adjoint_work_bytes(int n, int r, int n_terms, int F, bool own_lambda);
+// params: host copy of the parameter descriptors; X: the solutions, F blocks of n x r.
+cudaError_t launch_adjoint(const AdjointArgs &a, const DParamDev *params, const double2 *X, int n, int r, int F,
+                           void *work, int sms, double *dJdp, cudaStream_t st);
 
 }  // namespace srom

@@ -1107,7 +1107,8 @@ int srom_sweep_backward(srom_handle *h, const srom_rom_desc *rom, const srom_com
     const size_t o_term = o_par + align_up(sizeof(srom::DParamDev) * n_params, 256);
     const size_t o_ctr = o_term + align_up(sizeof(srom::DParamTerm) * std::max<size_t>(terms.size(), 1), 256);
     const size_t o_part = o_ctr + 256;
-    const size_t total = o_part + sizeof(double) * (size_t)rom->F * n_params;
+    const size_t o_work = o_part + align_up(sizeof(double) * (size_t)rom->F * n_params, 256);
+    const size_t total = o_work + srom::adjoint_work_bytes(rom->n, rom->r, (int)terms.size(), rom->F, !lambda);
     if (h->meta_pending) {
         SROM_CUDA(h, cudaEventSynchronize(h->meta_done));
         h->meta_pending = false;
@@ -1138,10 +1139,9 @@ int srom_sweep_backward(srom_handle *h, const srom_rom_desc *rom, const srom_com
     a.partial = reinterpret_cast<double *>(dm + o_part);
     a.lambda = reinterpret_cast<double2 *>(lambda);
     a.counter = reinterpret_cast<int *>(dm + o_ctr);
-    const int grid = std::min(rom->F, h->sm_count * 4);
     const double n3 = (double)rom->n * rom->n;
     ProfScope ps(h, "adjoint", rom->F, (8.0 * n3 * rom->r) * rom->F, 0.0);
-    SROM_CUDA(h, srom::launch_adjoint(a, rom->n, rom->r, rom->F, grid, dJdp, h->stream));
+    SROM_CUDA(h, srom::launch_adjoint(a, pd.data(), rd.X, rom->n, rom->r, rom->F, dm + o_work, h->sm_count, dJdp, h->stream));
     return SROM_OK;
 }
 
