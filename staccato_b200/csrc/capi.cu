@@ -361,8 +361,8 @@ namespace {
 // A validated, classified and ordered sweep: the host image of the device metadata
 // (descriptors, cost-ordered work lists, fallback list, zeroed counters) plus launch shapes.
 // Storage classes of a plan: 0 FP64 orders whose matrix fits shared memory (routed to the row
-// kernel), 1 global kernel (FP64 above n = 512, or the CUDA-core mixed kernel), 2 large-order FP64
-// kernel, 3 tensor-core mixed kernel, 4..7 the FP64 row kernel (sweep_lu64.cu) with 64, 128, 256
+// kernel), 1 FP64 above n = 512 or the CUDA-core mixed kernel, 2 FP64 of large orders (FP64 of both
+// classes: sweep_large.cu), 3 tensor-core mixed kernel, 4..7 the FP64 row kernel (sweep_lu64.cu) with 64, 128, 256
 // and 512 threads a system.
 constexpr int NCLS = 8;
 constexpr int CLS_ROW = 4, N_ROW = 4;
@@ -382,7 +382,7 @@ struct SweepPlan {
     int r_nmax[N_ROW] = {}, r_rmax[N_ROW] = {};  // classes 4..7
     long long grid1 = 0, grid2 = 0, grid3 = 0, gridr[N_ROW] = {}, gridf = 0;
     int64_t slot_bytes = 0, slot2_bytes = 0, slot3_bytes = 0, slotf_bytes = 0, slotr_bytes[N_ROW] = {};
-    bool need_scratch = false;
+    bool need_scratch = false, keep = false;  // keep: some system keeps its factors
     std::vector<srom::BackProj> backproj;  // ROMs whose solutions are projected onto outputs
     // ROMs without a mass matrix.  Their descriptors point M at a zero matrix instead: for any
     // finite w, K + (-w^2)*0 adds -0, which leaves every value (and the sign of zero) as it is,
@@ -540,6 +540,7 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
         if (cls[i] < 0) continue;
         if (d.n <= srom::LU64_MAX_N && (cls[i] == 0 || cls[i] == 2 || (cls[i] == 1 && !mixed)))
             cls[i] = CLS_ROW + row_class(d.n, cls[i] == 1 && srom::fp64_smem_bytes(d.n, d.r) <= smem_cap);
+        P.keep = P.keep || d.LU;
         const int c = cls[i];
         int *nm = c == 1 ? &P.g_nmax : c == 2 ? &P.b_nmax : c == 3 ? &P.t_nmax : &P.r_nmax[c - CLS_ROW];
         int *rm = c == 1 ? &P.g_rmax : c == 2 ? &P.b_rmax : c == 3 ? &P.t_rmax : &P.r_rmax[c - CLS_ROW];
@@ -560,10 +561,9 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
     }
     if (P.n_items[1] > 0) {
         P.grid1 = std::min<long long>(P.n_items[1], h->sm_count);
-        P.slot_bytes = (int64_t)P.g_nmax * P.g_nmax * (int64_t)sizeof(double2);
-        P.need_scratch = P.need_scratch || mixed;
-        for (int i = 0; i < n_roms; ++i)
-            if (cls[i] == 1 && !roms[i].LU) P.need_scratch = true;
+        P.slot_bytes = mixed ? (int64_t)P.g_nmax * P.g_nmax * (int64_t)sizeof(double2)
+                             : srom::large_slot_bytes(P.g_nmax, P.g_rmax);
+        P.need_scratch = true;
     }
     if (P.n_items[3] > 0) {
         P.grid3 = std::min<long long>(P.n_items[3], h->sm_count);
@@ -583,10 +583,10 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
             P.slotf_bytes = srom::big_slot_bytes(P.f_nmax);
     }
     if (P.n_items[2] > 0) {
-        // one system per CTA: matrix (or the caller's LU buffer) and the panel in the CTA's slot;
-        // classes 1 and 2 run one after the other and share the scratch buffer
+        // systems in flight, a slot each; classes 1 and 2 run one after the other and share the
+        // scratch buffer
         P.grid2 = std::min<long long>(P.n_items[2], h->sm_count);
-        P.slot2_bytes = srom::big_slot_bytes(P.b_nmax);
+        P.slot2_bytes = srom::large_slot_bytes(P.b_nmax, P.b_rmax);
         P.need_scratch = true;
     }
     // Work lists: largest systems first (longest-processing-time order for the persistent CTAs).
@@ -623,7 +623,7 @@ size_t plan_scratch_bytes(const SweepPlan &P) {
 
 // Counters live at off_ctr and must be zero when the launches start (the metadata copy zeroes
 // them, or zero_counters does): 1 global kernel, 2 fallback count, 3 fallback work, 4 tensor-core
-// error word, 5 large-order kernel, 6 tensor-core kernel, 8..11 row kernel.
+// error word, 6 tensor-core kernel, 8..11 row kernel.
 int enqueue_plan(srom_handle *h, const SweepPlan &P, char *dm, void *scratch, cudaStream_t st, bool zero_counters,
                  bool profile) {
     const RomDev *d_roms = reinterpret_cast<const RomDev *>(dm);
@@ -672,11 +672,25 @@ int enqueue_plan(srom_handle *h, const SweepPlan &P, char *dm, void *scratch, cu
         a.fb_count = fb_count;
         return a;
     };
+    auto large = [&](int c, long long group, int64_t slot, int n_max, int r_max) {
+        srom::LargeArgs a{};
+        a.roms = d_roms;
+        a.items = items(c);
+        a.n_items = (int)P.n_items[c];
+        a.group = (int)group;
+        a.scratch = static_cast<unsigned char *>(scratch);
+        a.slot_bytes = slot;
+        a.n_max = n_max;
+        a.r_max = r_max;
+        a.sms = h->sm_count;
+        a.keep = P.keep;
+        return srom::launch_large(a, st);
+    };
     if (rc == SROM_OK && P.n_items[1] > 0) {
-        srom::GlobalArgs a = mixed_args(1, d_ctr + 1, P.slot_bytes, P.g_nmax, P.g_rmax);
-        if (!P.mixed) a.fb_items = nullptr, a.fb_count = nullptr;
         ProfScope ps(h, P.mixed ? "mixed_global" : "fp64_global", P.n_items[1], P.flops[1], 0.0);
-        cudaError_t e = srom::launch_global(P.mixed, a, (int)P.grid1, st);
+        cudaError_t e = P.mixed ? srom::launch_global(true, mixed_args(1, d_ctr + 1, P.slot_bytes, P.g_nmax, P.g_rmax),
+                                                      (int)P.grid1, st)
+                                : large(1, P.grid1, P.slot_bytes, P.g_nmax, P.g_rmax);
         if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "global launch: %s", cudaGetErrorString(e));
     }
     if (rc == SROM_OK && P.n_items[3] > 0) {
@@ -708,17 +722,8 @@ int enqueue_plan(srom_handle *h, const SweepPlan &P, char *dm, void *scratch, cu
         if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "fallback launch: %s", cudaGetErrorString(e));
     }
     if (rc == SROM_OK && P.n_items[2] > 0) {
-        srom::GlobalArgs a{};
-        a.roms = d_roms;
-        a.items = items(2);
-        a.n_items = (int)P.n_items[2];
-        a.counter = d_ctr + 5;
-        a.scratch = static_cast<unsigned char *>(scratch);
-        a.slot_bytes = P.slot2_bytes;
-        a.n_max = P.b_nmax;
-        a.r_max = P.b_rmax;
         ProfScope ps(h, "fp64_large", P.n_items[2], P.flops[2], 0.0);
-        cudaError_t e = srom::launch_global_big(a, (int)P.grid2, st);
+        cudaError_t e = large(2, P.grid2, P.slot2_bytes, P.b_nmax, P.b_rmax);
         if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "large-order launch: %s", cudaGetErrorString(e));
     }
     for (size_t i = 0; rc == SROM_OK && i < P.backproj.size(); ++i) {

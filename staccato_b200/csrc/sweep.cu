@@ -9,8 +9,9 @@
 // physically moved while the column is being searched.  After the panel, every warp independently
 // processes its own groups of CW trailing columns: apply the panel's interchanges, solve the
 // unit-lower triangle for the U rows (warp shuffles), and update the remaining rows with
-// register-tiled complex FMAs.  No CTA barrier separates the column groups.  FP64 systems of orders up
-// to 512 run on the row kernel of sweep_lu64.cu instead.
+// register-tiled complex FMAs.  No CTA barrier separates the column groups.  FP64 sweeps run on
+// sweep_lu64.cu (orders up to 512) and sweep_large.cu (above); the FP64 instances here re-solve the
+// mixed form's non-converged systems of orders above 512, whose number only the device knows.
 //
 // Precision forms
 //   FP64  (double2): reproduces LAPACK zgetrf/zgetrs as restated in the oracle bit for bit:
@@ -679,10 +680,7 @@ cudaError_t launch_global_big(const GlobalArgs &a0, int grid, cudaStream_t st) {
     if (a.slot_bytes < big_slot_bytes(a.n_max)) return cudaErrorInvalidValue;
     a.panel_off = big_panel_offset(a.n_max);
     const int rpt = global_rpt(a.n_max);
-    if (rpt <= 3) return launch_global_t<false, 3, true>(a, grid, st);
-    if (rpt <= 6) return launch_global_t<false, 6, true>(a, grid, st);
-    if (rpt <= BIG_RPT) return launch_global_t<false, BIG_RPT, true>(a, grid, st);
-    return cudaErrorInvalidValue;
+    return rpt <= GLOBAL_MAX_RPT ? launch_global_t<false, GLOBAL_MAX_RPT, true>(a, grid, st) : cudaErrorInvalidValue;
 }
 
 }  // namespace srom

@@ -26,8 +26,7 @@ size_t global_smem_bytes(int n_max, int r_max, bool big = false);
 bool global_panel_fits(int n_max, int r_max, int smem_optin);
 int global_rpt(int n_max);
 constexpr int GLOBAL_MAX_RPT = 3;   // rows per thread of the shared-memory-panel instances
-constexpr int BIG_RPT = 10;         // the largest large-order FP64 instance: n <= NT * BIG_RPT = 2560
-constexpr int BIG_MAX_N = 256 * BIG_RPT;
+constexpr int BIG_MAX_N = 2560;     // the largest order of all
 // large-order FP64 instance: global scratch per CTA (the matrix, then the 16-column panel)
 int64_t big_panel_offset(int n_max);
 int64_t big_slot_bytes(int n_max);
@@ -54,8 +53,8 @@ struct GlobalArgs {
 };
 // Global-storage kernel, FP64 (mixed = false) or complex-FP32 factors + FP64 refinement.
 cudaError_t launch_global(bool mixed, const GlobalArgs &a, int grid, cudaStream_t st);
-// FP64 sweep of orders up to BIG_MAX_N with the panel in global scratch (slot_bytes >=
-// big_slot_bytes(n_max)); 3, 6 or 10 rows per thread by n_max
+// The same with the FP64 panel in global scratch (slot_bytes >= big_slot_bytes(n_max)): systems up to
+// n = 768 whose panel and right-hand sides do not fit shared memory together
 cudaError_t launch_global_big(const GlobalArgs &a, int grid, cudaStream_t st);
 
 // ---- FP64, orders up to LU64_MAX_N (sweep_lu64.cu): one thread a row, Schur updates on the FP64
@@ -64,6 +63,22 @@ constexpr int LU64_MAX_N = 512;
 int lu64_blocks_per_sm(int threads, int n_max);
 int64_t lu64_slot_bytes(int n_max, int r_max);  // global scratch per CTA
 cudaError_t launch_lu64(int threads, const GlobalArgs &a, int grid, cudaStream_t st);
+
+// ---- FP64, large orders (sweep_large.cu): groups of systems advance panel by panel, several
+// multiprocessors a system; a sequence of launches on the stream ----
+constexpr int LARGE_MAX_N = BIG_MAX_N;
+struct LargeArgs {
+    const RomDev *roms;
+    const Item *items;
+    int n_items;
+    int group;               // systems in flight: scratch holds group slots
+    unsigned char *scratch;
+    int64_t slot_bytes;      // at least large_slot_bytes(n_max, r_max)
+    int n_max, r_max, sms;
+    bool keep;               // some system keeps its factors
+};
+int64_t large_slot_bytes(int n_max, int r_max);
+cudaError_t launch_large(const LargeArgs &a, cudaStream_t st);
 
 // ---- tensor-core mixed form (sweep_tc.cu): complex-FP32 LU whose Schur updates run as
 // tcgen05 MMAs on three-piece bf16 splits, FP64 refinement as in the global kernel ----
