@@ -11,10 +11,12 @@
 //                 band is a column-major matrix with leading dimension ldab-1;
 //  * factor    -- blocked LDL^T without pivoting (K~ is complex symmetric), NB columns a step:
 //                 the NB x NB diagonal block in one CTA, the panel L21 = A21 L11^-T D^-1 by one
-//                 warp a row, and the trailing update A22 -= (L21 D) L21^T as one strided-batched
-//                 complex GEMM over the column blocks of the window (zgemm.cu, FP64 tensor cores);
-//  * solves    -- blocked forward / diagonal / backward substitution for all right-hand sides,
-//                 the off-diagonal block updates as complex GEMMs (split over k when short and wide).
+//                 warp a row, and the trailing update A22 -= (L21 D) L21^T of the window's lower
+//                 triangle on the FP64 tensor cores, the next diagonal block and panel running on a
+//                 side stream meanwhile;
+//  * solves    -- blocked forward / diagonal / backward substitution, one launch a block for up to 16
+//                 right-hand sides; for more, the off-diagonal block updates as complex GEMMs (split
+//                 over k when short and wide).
 //
 // The rest of the process runs on the GPU as in the reference: M Q by a complex CSR SpMM, the
 // re-orthogonalisation Q <- Q - V (V^H Q) with complex GEMMs (V^H Q split over the rows, reduced
@@ -108,11 +110,7 @@ __global__ void scatter_band_kernel(int64_t n, const int64_t *__restrict__ rp, c
 
 // ---- blocked LDL^T ------------------------------------------------------------------------
 // The nb x nb diagonal block at column j0: A11 = L11 D L11^T (unit L11, no pivoting), in place
-// (D on the diagonal).  The block is held whole (both triangles) in shared memory; step k
-// updates a_ij -= a_ik (a_kj / d_k) for i, j > k, each thread owning one column j (its row
-// entries are contiguous across the warp) and every fourth row, so a step needs one barrier.
-// The columns are scaled by 1/d_k once at the end.  The first exactly-zero pivot is recorded
-// 1-based in *info.
+// (D on the diagonal).  The first exactly-zero pivot is recorded 1-based in *info.
 // Small pivots are perturbed as PARDISO does with the reference's setting iparm[9] = 13
 // (KrylovROMSubstructure.cpp:621): a pivot d with |d| < 1e-13 ||A||_inf is replaced by the value
 // of the same phase and modulus 1e-13 ||A||_inf, and counted in *perturbed; *min_ratio_bits
@@ -126,46 +124,87 @@ __device__ __forceinline__ double2 perturb_pivot(double2 d, double tau) {
     return make_double2(d.x * s, d.y * s);
 }
 
+// One CTA.  Thread (ti, tj) of a 16 x 16 grid holds entries (ti + 16 a, tj + 16 b) of the whole symmetric
+// block in registers.  Step k: the owners of row and column k have published them in shared memory (two
+// buffers) and every thread subtracts a_ik (a_kj / d_k): one barrier a step, a chain of 64 steps of about
+// 0.2 us (61 us a block when the block lived in shared memory and every thread evaluated the pivot's
+// modulus).  The moduli for the statistics are taken once, after the last step.
 __global__ void __launch_bounds__(KT) ldlt_diag_kernel(double2 *__restrict__ band, int64_t ldab, int64_t j0, int nb,
                                                        int *__restrict__ info,
                                                        const unsigned long long *__restrict__ anorm_bits,
                                                        int *__restrict__ perturbed,
                                                        unsigned long long *__restrict__ min_ratio_bits) {
-    extern __shared__ double2 S[];  // S[i * SLD + j], full symmetric block
-    constexpr int RS = KT / NB;     // row stride of a thread
-    const int t = threadIdx.x;
+    static_assert(KT == 256 && NB == 64, "a 16 x 16 thread grid of 4 x 4 entries");
+    __shared__ double2 col[2][NB], row[2][NB];
+    __shared__ double2 piv[NB];  // the pivots before perturbation
+    const int t = threadIdx.x, ti = t & 15, tj = t >> 4;
     const double anorm = __longlong_as_double((long long)*anorm_bits);
     const double tau = PIVOT_EPS * anorm;
-    for (int e = t; e < nb * nb; e += KT) {
-        const int i = e / nb, j = e % nb;
-        const int r = max(i, j), c = min(i, j);
-        S[i * SLD + j] = band[(j0 + c) * ldab + (r - c + NB)];
+    double2 v[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int i = ti + 16 * a, j = tj + 16 * b, r = max(i, j), c = min(i, j);
+            v[a][b] = r < nb ? band[(j0 + c) * ldab + (r - c + NB)] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        if (tj == 0) col[0][ti + 16 * a] = v[a][0];
+        if (ti == 0) row[0][tj + 16 * a] = v[0][a];
     }
     __syncthreads();
-    const int j = t % NB, ir = t / NB;
-    for (int k = 0; k < nb; ++k) {
-        const double2 d0 = S[k * SLD + k];
-        const double2 d = perturb_pivot(d0, tau);  // the same value in every thread
-        if (t == 0) {
-            if (d0.x == 0.0 && d0.y == 0.0) atomicCAS(info, 0, (int)(j0 + k + 1));
-            const double a = hypot(d0.x, d0.y);
-            if (a < tau) atomicAdd(perturbed, 1);
-            if (anorm > 0.0) atomicMin(min_ratio_bits, (unsigned long long)__double_as_longlong(a / anorm));
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {  // columns 16 g .. 16 g + 15
+        for (int kk = 0; kk < 16; ++kk) {
+            const int k = 16 * g + kk;
+            if (k >= nb) break;
+            const double2 *c = col[k & 1];
+            const double2 d0 = c[k];
+            double2 d = d0;
+            // max(|re|, |im|) >= tau implies |d| >= tau
+            if (!(fmax(fabs(d0.x), fabs(d0.y)) >= tau)) d = perturb_pivot(d0, tau);
+            const double2 inv = crecip(d);
+            double2 ri[4], cj[4];
+#pragma unroll
+            for (int a = g; a < 4; ++a) {
+                ri[a] = c[ti + 16 * a];
+                cj[a] = cmul(row[k & 1][tj + 16 * a], inv);
+            }
+            if (t < NB && t >= k && t < nb) band[(j0 + k) * ldab + (t - k + NB)] = t == k ? d : cmul(c[t], inv);
+            if (t == k) piv[k] = d0;
+#pragma unroll
+            for (int b = g; b < 4; ++b)
+#pragma unroll
+                for (int a = g; a < 4; ++a)
+                    if (ti + 16 * a > k && tj + 16 * b > k) v[a][b] = cfms(v[a][b], ri[a], cj[b]);
+            // row and column k + 1, from their owners
+#pragma unroll
+            for (int b = g; b < 4; ++b) {
+                if (k + 1 == tj + 16 * b) {
+#pragma unroll
+                    for (int a = g; a < 4; ++a) col[(k + 1) & 1][ti + 16 * a] = v[a][b];
+                }
+                if (k + 1 == ti + 16 * b) {
+#pragma unroll
+                    for (int a = g; a < 4; ++a) row[(k + 1) & 1][tj + 16 * a] = v[b][a];
+                }
+            }
+            __syncthreads();
         }
-        if (j > k && j < nb) {
-            const double2 cj = cmul(S[k * SLD + j], crecip(d));
-            for (int i = k + 1 + ((ir - (k + 1)) % RS + RS) % RS; i < nb; i += RS)
-                S[i * SLD + j] = cfms(S[i * SLD + j], S[i * SLD + k], cj);
-        }
-        __syncthreads();
     }
-    for (int e = t; e < nb * nb; e += KT) {
-        const int i = e % nb, c = e / nb;
-        const double2 dc = perturb_pivot(S[c * SLD + c], tau);  // step c never changes S[c][c]
-        if (i > c)
-            band[(j0 + c) * ldab + (i - c + NB)] = cmul(S[i * SLD + c], crecip(dc));
-        else if (i == c)
-            band[(j0 + c) * ldab + NB] = dc;
+    __shared__ unsigned zero[2];
+    if (t < NB) {
+        const unsigned z = __ballot_sync(0xffffffffu, t < nb && piv[t].x == 0.0 && piv[t].y == 0.0);
+        if ((t & 31) == 0) zero[t >> 5] = z;
+    }
+    __syncthreads();
+    if (t == 0 && (zero[0] | zero[1])) atomicCAS(info, 0, (int)(j0 + (zero[0] ? __ffs(zero[0]) : 32 + __ffs(zero[1]))));
+    if (t < nb) {
+        const double2 d0 = piv[t];
+        const double m = hypot(d0.x, d0.y);
+        if (m < tau) atomicAdd(perturbed, 1);
+        if (anorm > 0.0) atomicMin(min_ratio_bits, (unsigned long long)__double_as_longlong(m / anorm));
     }
 }
 
@@ -179,12 +218,10 @@ __device__ __forceinline__ void load_l11(const double2 *band, int64_t ldab, int6
 }
 
 // Panel rows t in [0, rows) (matrix rows j0+nb+t): x L11^T = a, L21 = x D^-1; x goes to W
-// (= L21 D) and L21 to Lp and to the band.  Rows [rows, zero_to) of W and Lp are zeroed (the
-// strided-batched update reads up to NB * (batches - 1) + rows rows).  One warp a row, lane l
-// holding columns l and l + 32.
+// (= L21 D) and L21 to Lp and to the band.  One warp a row, lane l holding columns l and l + 32.
 __global__ void __launch_bounds__(KT) ldlt_panel_kernel(double2 *__restrict__ band, int64_t ldab, int64_t j0, int nb,
-                                                        int rows, int zero_to, double2 *__restrict__ W,
-                                                        double2 *__restrict__ Lp, int ldw) {
+                                                        int rows, double2 *__restrict__ W, double2 *__restrict__ Lp,
+                                                        int ldw) {
     extern __shared__ double2 S[];  // L11 (NB x SLD) then 1/d (NB)
     double2 *Dinv = S + NB * SLD;
     load_l11(band, ldab, j0, nb, S);
@@ -192,14 +229,7 @@ __global__ void __launch_bounds__(KT) ldlt_panel_kernel(double2 *__restrict__ ba
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int t = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    if (t >= zero_to) return;
-    if (t >= rows) {
-        for (int k = lane; k < NB; k += 32) {
-            W[t + (int64_t)k * ldw] = make_double2(0.0, 0.0);
-            Lp[t + (int64_t)k * ldw] = make_double2(0.0, 0.0);
-        }
-        return;
-    }
+    if (t >= rows) return;
     const int64_t r = j0 + nb + t;
     double2 x[2];
 #pragma unroll
@@ -228,6 +258,330 @@ __global__ void __launch_bounds__(KT) ldlt_panel_kernel(double2 *__restrict__ ba
             W[t + (int64_t)k * ldw] = wv;
             Lp[t + (int64_t)k * ldw] = l;
         }
+    }
+}
+
+// ---- trailing update -----------------------------------------------------------------------
+// A22 -= W Lp^T on the lower triangle of the window (rows x rows, the band addressed as a dense matrix of
+// leading dimension ldab - 1): a CTA a tile of 64 rows of one 64-column block, k = 64 in four chunks of 16
+// through a three-deep cp.async ring, warp w on columns 16 (w & 3) .. + 15 and 32 of the rows.  The product is
+// summed as zgemm.cu sums it (4M, chunks of four k, real by real before imaginary by imaginary) and then
+// subtracted, so the factor's bits are those of the strided-batched GEMM that did this before: over whole
+// columns of the window, the upper half computed and thrown away, 0.22 ms an update on the Tet10 block
+// (bw = 2876); this kernel takes 0.10 ms (0.083 and 0.016 for the first column block).
+constexpr int UP_T = 256, UP_KC = 16, UP_NC = NB / UP_KC, UP_STAGES = 3;
+constexpr int UP_LD = 64 + 2;  // 2 modulo 8: the four k rows of a fragment load fall in different banks
+constexpr size_t UP_SMEM = sizeof(double2) * 2 * UP_KC * UP_LD * UP_STAGES;
+
+__device__ __forceinline__ void cp16(double2 *dst, const double2 *src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
+}
+__device__ __forceinline__ void dmma(double2 &c, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(c.x), "+d"(c.y)
+        : "d"(a), "d"(b));
+}
+
+__global__ void __launch_bounds__(UP_T, 2) ldlt_update_kernel(double2 *__restrict__ C0, int64_t ldc, const double2 *__restrict__ W,
+                                                              const double2 *__restrict__ Lp, int ldw, int rows, int jb0) {
+    extern __shared__ double2 S[];
+    const int cb = (jb0 + (int)blockIdx.y) * NB, r0 = cb + (int)blockIdx.x * 64;
+    if (r0 >= rows) return;
+    const int nr = min(64, rows - r0), nc = min(64, rows - cb);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto stage = [&](int ch) {
+        if (ch < UP_NC) {
+            double2 *SA = S + (ch % UP_STAGES) * 2 * UP_KC * UP_LD, *SB = SA + UP_KC * UP_LD;
+            for (int e = tid; e < UP_KC * 64; e += UP_T) {
+                const int i = e & 63, k = e >> 6;
+                const int64_t kk = (int64_t)(ch * UP_KC + k) * ldw;
+                if (i < nr) cp16(SA + k * UP_LD + i, W + r0 + i + kk);
+                if (i < nc) cp16(SB + k * UP_LD + i, Lp + cb + i + kk);
+            }
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+    stage(0);
+    stage(1);
+    const int strip = warp & 3, half = warp >> 2;
+    const int lr = lane >> 2, lk = lane & 3;
+    double2 re[4][2], im[4][2];  // [8-row tile][column tile]: components of the two columns
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) re[x][y] = im[x][y] = make_double2(0.0, 0.0);
+    for (int ch = 0; ch < UP_NC; ++ch) {
+        asm volatile("cp.async.wait_group 1;");
+        __syncthreads();  // chunk ch is in; everyone is done with chunk ch - 1's buffer
+        stage(ch + 2);
+        const double2 *pa = S + (ch % UP_STAGES) * 2 * UP_KC * UP_LD + lk * UP_LD + half * 32 + lr;
+        const double2 *pb = S + ((ch % UP_STAGES) * 2 + 1) * UP_KC * UP_LD + lk * UP_LD + strip * 16 + lr;
+#pragma unroll
+        for (int k = 0; k < UP_KC; k += 4) {
+            double2 va[4], vb[2];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) va[x] = pa[k * UP_LD + 8 * x];
+#pragma unroll
+            for (int y = 0; y < 2; ++y) vb[y] = pb[k * UP_LD + 8 * y];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    dmma(re[x][y], va[x].x, vb[y].x);
+                    dmma(im[x][y], va[x].x, vb[y].y);
+                }
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    dmma(re[x][y], -va[x].y, vb[y].y);
+                    dmma(im[x][y], va[x].y, vb[y].x);
+                }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;");
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int cc = strip * 16 + 8 * y + 2 * lk + h;
+            if (cc >= nc) continue;
+            double2 *c = C0 + r0 + (int64_t)(cb + cc) * ldc + half * 32 + lr;
+            double2 old[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+                if (half * 32 + 8 * x + lr < nr) old[x] = c[8 * x];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+                if (half * 32 + 8 * x + lr < nr)
+                    c[8 * x] = make_double2(old[x].x - (h ? re[x][y].y : re[x][y].x), old[x].y - (h ? im[x][y].y : im[x][y].x));
+        }
+}
+
+// ---- substitution, few right-hand sides ----------------------------------------------------
+// One launch a 64-row block, r <= SOLVE_RMAX right-hand sides.  The sums are taken in the order of the complex
+// GEMMs that serve more right-hand sides (gemm_term: chunks of four k, real by real first; over the long sums
+// of the backward direction, the GEMM's split into chunks of kchunk rows, added up in order), so both routes
+// give the same bits.  On the Tet10 block with four right-hand sides a block step takes 15 us forward and 17 us
+// backward (a launch measured alone), against 29 and 35 us as two or three launches.
+constexpr int SOLVE_RMAX = 16, SOLVE_LDT = NB + 1;
+
+// acc += sum of l[k] x[k] over four k (k0 + 4 <= kn or the tail, where missing terms are zeros)
+__device__ __forceinline__ void gemm_terms(double2 &acc, const double2 (&l)[4], const double2 (&x)[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        acc.x = fma(l[k].x, x[k].x, acc.x);
+        acc.y = fma(l[k].x, x[k].y, acc.y);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        acc.x = fma(-l[k].y, x[k].y, acc.x);
+        acc.y = fma(l[k].y, x[k].x, acc.y);
+    }
+}
+
+// A block step depends on the one before it only through the right-hand sides: its launch may start while
+// the other still runs (programmatic stream serialisation), fetches its part of L and waits here.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The unit lower triangle of block j0 into shared memory, S[k * SOLVE_LDT + i] = L[i][k], i > k.
+__device__ __forceinline__ void fetch_l11(const double2 *band, int64_t ldab, int64_t j0, int nb, double2 *S) {
+    for (int k = threadIdx.x >> 5; k < nb; k += KT / 32)
+        for (int i = threadIdx.x & 31; i < nb; i += 32)
+            if (i > k) cp16(S + k * SOLVE_LDT + i, band + (j0 + k) * ldab + (i - k + NB));
+    asm volatile("cp.async.commit_group;");
+}
+
+// L11 y = v or L11^T y = v by one warp, lane l holding rows l and l + 32 (trsv_block_kernel's order).
+template <bool BACK>
+__device__ __forceinline__ void solve_l11(const double2 *S, int nb, double2 (&v)[2]) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (!BACK) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+            for (int m = 32 * g; m < min(nb, 32 * g + 32); ++m) {
+                const double2 vm = shfl2(v[g], m & 31);
+#pragma unroll
+                for (int h = g; h < 2; ++h) {
+                    const int k = lane + 32 * h;
+                    if (k > m && k < nb) v[h] = cfms(v[h], S[m * SOLVE_LDT + k], vm);
+                }
+            }
+    } else {
+#pragma unroll
+        for (int g = 1; g >= 0; --g)
+            for (int m = min(nb, 32 * g + 32) - 1; m >= 32 * g; --m) {
+                const double2 vm = shfl2(v[g], m & 31);
+#pragma unroll
+                for (int h = 0; h <= g; ++h) {
+                    const int k = lane + 32 * h;
+                    if (k < m) v[h] = cfms(v[h], S[k * SOLVE_LDT + m], vm);
+                }
+            }
+    }
+}
+
+// Forward: y = L11^-1 x_k in every CTA (one warp a right-hand side), then x_i -= L[i, k] y for the CTA's 64
+// rows, whose tile of L has been fetched meanwhile (a thread a row and right-hand side).  CTA 0
+// stores y / D into dst, another array than src: the other CTAs may still read x_k.
+__host__ __device__ constexpr size_t forward_smem(int r) { return sizeof(double2) * (2 * NB * SOLVE_LDT + NB * r); }
+
+__global__ void __launch_bounds__(KT) solve_forward_kernel(const double2 *__restrict__ band, int64_t ldab, int64_t j0, int nb,
+                                                           int rows, double2 *__restrict__ src, int64_t lds,
+                                                           double2 *__restrict__ dst, int64_t ldd, int r) {
+    extern __shared__ double2 sh[];
+    double2 *L11 = sh, *T = L11 + NB * SOLVE_LDT, *Y = T + NB * SOLVE_LDT;  // T[k][i]: row i of the CTA's tile
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int w0 = (int)blockIdx.x * NB, nt = min(NB, rows - w0);
+    const int64_t i0 = j0 + nb + w0;
+    let_next_start();
+    fetch_l11(band, ldab, j0, nb, L11);
+    for (int k = warp; k < nb; k += KT / 32)
+        for (int i = lane; i < nt; i += 32) cp16(T + k * SOLVE_LDT + i, band + (j0 + k) * ldab + (i0 + i - (j0 + k) + NB));
+    asm volatile("cp.async.commit_group;");
+    wait_for_previous();
+    asm volatile("cp.async.wait_group 1;");
+    __syncthreads();
+    for (int c = warp; c < r; c += KT / 32) {
+        const double2 *x = src + (int64_t)c * lds + j0;
+        double2 v[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) v[h] = lane + 32 * h < nb ? x[lane + 32 * h] : make_double2(0.0, 0.0);
+        solve_l11<false>(L11, nb, v);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = lane + 32 * h;
+            if (k < nb) {
+                Y[k + c * NB] = v[h];
+                if (blockIdx.x == 0) dst[(int64_t)c * ldd + j0 + k] = cdiv(v[h], band[(j0 + k) * ldab + NB]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;");
+    __syncthreads();
+    const int i = tid & 63;  // rows below the block exist only for a full one: nb = 64 here
+    for (int c = tid >> 6; c < r && i < nt; c += KT / 64) {
+        double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int k = 0; k < NB; k += 4) {
+            double2 l[4], y[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                l[q] = T[(k + q) * SOLVE_LDT + i];
+                y[q] = Y[k + q + c * NB];
+            }
+            gemm_terms(acc, l, y);
+        }
+        double2 &x = src[(int64_t)c * lds + i0 + i];
+        x = make_double2(x.x - acc.x, x.y - acc.y);
+    }
+}
+
+// Backward: CTA s sums L[i, k]^T x_i over the rows [s kchunk, (s + 1) kchunk) below the block (a thread a
+// column of the block and right-hand side, four rows at a time from shared memory) into part; the CTA that
+// finishes last (a ticket, no waiting) adds the chunks up in order, subtracts them from y_k and solves
+// L11^T x = y_k in place.
+constexpr int BACK_TR = 72;  // rows staged at a time
+__host__ __device__ constexpr size_t backward_smem(int r) { return sizeof(double2) * (NB * (BACK_TR + 1) + BACK_TR * r); }
+static_assert(SOLVE_LDT <= BACK_TR + 1 && NB <= BACK_TR, "the triangle and the right-hand sides fit the tile's place");
+
+__global__ void __launch_bounds__(KT) solve_backward_kernel(const double2 *__restrict__ band, int64_t ldab, int64_t j0, int nb,
+                                                            int rows, int kchunk, double2 *__restrict__ X, int64_t ldx, int r,
+                                                            double2 *__restrict__ part, unsigned *__restrict__ ticket) {
+    extern __shared__ double2 sh[];
+    __shared__ bool last;
+    double2 *T = sh, *Xs = T + NB * (BACK_TR + 1);  // T[k][i]: L[i][k]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int splits = (int)gridDim.x, s = (int)blockIdx.x;
+    const int k = tid & 63;
+    let_next_start();
+    if (rows <= 0) wait_for_previous();
+    if (rows > 0) {
+        double2 acc[SOLVE_RMAX / (KT / 64)];
+#pragma unroll
+        for (int q = 0; q < SOLVE_RMAX / (KT / 64); ++q) acc[q] = make_double2(0.0, 0.0);
+        const int beg = min(s * kchunk, rows), end = min(beg + kchunk, rows);
+        for (int b = beg; b < end; b += BACK_TR) {
+            const int nt = min(BACK_TR, end - b), np = (nt + 3) & ~3;
+            __syncthreads();
+            for (int c = warp; c < nb; c += KT / 32)
+                for (int i = lane; i < np; i += 32) {
+                    double2 *d = T + c * (BACK_TR + 1) + i;
+                    if (i < nt) cp16(d, band + (j0 + c) * ldab + (nb + b + i - c + NB));
+                    else *d = make_double2(0.0, 0.0);
+                }
+            if (b == beg) wait_for_previous();
+            for (int c = warp; c < r; c += KT / 32)
+                for (int i = lane; i < np; i += 32) {
+                    double2 *d = Xs + c * BACK_TR + i;
+                    if (i < nt) cp16(d, X + (int64_t)c * ldx + j0 + nb + b + i);
+                    else *d = make_double2(0.0, 0.0);
+                }
+            asm volatile("cp.async.commit_group;");
+            asm volatile("cp.async.wait_group 0;");
+            __syncthreads();
+            if (k < nb)
+#pragma unroll
+                for (int q = 0; q < SOLVE_RMAX / (KT / 64); ++q) {
+                    const int c = (tid >> 6) + q * (KT / 64);
+                    if (c >= r) break;
+                    for (int i = 0; i < np; i += 4) {
+                        double2 l[4], x[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            l[u] = T[k * (BACK_TR + 1) + i + u];
+                            x[u] = Xs[c * BACK_TR + i + u];
+                        }
+                        gemm_terms(acc[q], l, x);
+                    }
+                }
+        }
+        if (beg >= end) wait_for_previous();  // part is still read by the step before
+        if (k < nb)
+#pragma unroll
+            for (int q = 0; q < SOLVE_RMAX / (KT / 64); ++q) {
+                const int c = (tid >> 6) + q * (KT / 64);
+                if (c < r) part[((int64_t)s * r + c) * NB + k] = acc[q];
+            }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) last = atomicAdd(ticket, 1u) == (unsigned)splits - 1;
+        __syncthreads();
+        if (!last) return;
+        if (tid == 0) *ticket = 0;  // for the next launch
+        __threadfence();
+    }
+    // the triangle and y_k less the chunks' sums take the place of the tile
+    double2 *Z = sh + NB * SOLVE_LDT;  // NB x r
+    fetch_l11(band, ldab, j0, nb, sh);
+    for (int e = tid; e < NB * r; e += KT) {
+        const int kk = e & (NB - 1), c = e / NB;
+        if (kk >= nb) continue;
+        double2 v = X[(int64_t)c * ldx + j0 + kk];
+        if (rows > 0) {
+            double2 sum = make_double2(0.0, 0.0);
+#pragma unroll 8
+            for (int u = 0; u < splits; ++u) {
+                const double2 p = __ldcg(part + ((int64_t)u * r + c) * NB + kk);
+                sum.x += p.x;
+                sum.y += p.y;
+            }
+            v = make_double2(v.x - sum.x, v.y - sum.y);
+        }
+        Z[e] = v;
+    }
+    asm volatile("cp.async.wait_group 0;");
+    __syncthreads();
+    for (int c = warp; c < r; c += KT / 32) {
+        double2 v[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) v[h] = lane + 32 * h < nb ? Z[c * NB + lane + 32 * h] : make_double2(0.0, 0.0);
+        solve_l11<true>(sh, nb, v);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (lane + 32 * h < nb) X[(int64_t)c * ldx + j0 + lane + 32 * h] = v[h];
     }
 }
 
@@ -596,7 +950,9 @@ struct BandLDLT {
     int ldw = 0;
     double2 *band = nullptr, *W = nullptr, *Lp = nullptr;
     int *d_info = nullptr;
-    cudaStream_t st = nullptr;
+    unsigned *d_ticket = nullptr;  // of solve_backward_kernel, zero between launches
+    cudaStream_t st = nullptr, side = nullptr;  // side: the look-ahead's diagonal blocks and panels
+    cudaEvent_t ev_panel = nullptr, ev_rest = nullptr;
     double2 *zwork = nullptr;  // split-k partials of the complex GEMMs
     int64_t zwork_elems = 0;
     int sms = 148;
@@ -634,27 +990,35 @@ struct BandLDLT {
         KCU(cudaMemsetAsync(d_info, 0, sizeof(int), st));
         KCU(cudaMemsetAsync(d_pert, 0, sizeof(int), st));
         KCU(cudaMemcpyAsync(d_minr, &inf_bits, sizeof inf_bits, cudaMemcpyHostToDevice, st));
-        int prev_rows = ldw;
-        for (int64_t j0 = 0; j0 < n; j0 += NB) {
+        // Look-ahead: the next step's diagonal block and panel need only the first column block of this
+        // step's update.  They run on the side stream, one step ahead of the rest of the update on st:
+        //   side: diag(k), panel(k), [rest(k-1)] first column block of update(k), diag(k+1), ...
+        //   st:   [panel(k)] rest(k), ...
+        // W and Lp alternate between two sets: panel(k + 1) writes one while rest(k) reads the other, and
+        // panel(k + 2) comes after the first block of update(k + 1), which has waited for rest(k).
+        KCU(cudaEventRecord(ev_rest, st));
+        KCU(cudaStreamWaitEvent(side, ev_rest, 0));
+        int step = 0;
+        for (int64_t j0 = 0; j0 < n; j0 += NB, ++step) {
             const int nb = (int)std::min<int64_t>(NB, n - j0);
-            ldlt_diag_kernel<<<1, KT, smem, st>>>(band, ldab, j0, nb, d_info, d_anorm, d_pert, d_minr);
+            ldlt_diag_kernel<<<1, KT, 0, side>>>(band, ldab, j0, nb, d_info, d_anorm, d_pert, d_minr);
             const int rows = (int)std::min<int64_t>(bw, n - j0 - nb);
             if (rows <= 0) continue;
-            const int zero_to = std::max(rows, prev_rows);
-            prev_rows = rows;
-            ldlt_panel_kernel<<<(zero_to + KT / 32 - 1) / (KT / 32), KT, smem + sizeof(double2) * NB, st>>>(
-                band, ldab, j0, nb, rows, zero_to, W, Lp, ldw);
-            // trailing update of the window: column block b (NB columns) -= W_b Lp_b^T, with
-            // W_b, Lp_b the panel rows from b NB on
-            const int batches = (rows + NB - 1) / NB;
+            double2 *Wk = W + (int64_t)(step & 1) * ldw * NB, *Lk = Lp + (int64_t)(step & 1) * ldw * NB;
+            ldlt_panel_kernel<<<(rows + KT / 32 - 1) / (KT / 32), KT, smem + sizeof(double2) * NB, side>>>(
+                band, ldab, j0, nb, rows, Wk, Lk, ldw);
+            KCU(cudaEventRecord(ev_panel, side));
+            KCU(cudaStreamWaitEvent(side, ev_rest, 0));  // rest(k - 1)
+            const int nblk = (rows + NB - 1) / NB;
             double2 *C0 = band + (j0 + nb) * ldab + NB;
-            Zgemm z = gemm(ZG_N, ZG_T, rows, NB, nb, W, ldw, Lp, ldw, C0, ldab - 1);
-            z.sa = NB;
-            z.sb = NB;
-            z.sc = (int64_t)NB * ldab;
-            z.batch = batches;
-            KCU(zgemm(z, st));
+            ldlt_update_kernel<<<dim3(nblk, 1), UP_T, UP_SMEM, side>>>(C0, ldab - 1, Wk, Lk, ldw, rows, 0);
+            KCU(cudaStreamWaitEvent(st, ev_panel, 0));
+            if (nblk > 1)
+                ldlt_update_kernel<<<dim3(nblk - 1, nblk - 1), UP_T, UP_SMEM, st>>>(C0, ldab - 1, Wk, Lk, ldw, rows, 1);
+            KCU(cudaEventRecord(ev_rest, st));
         }
+        KCU(cudaEventRecord(ev_panel, side));
+        KCU(cudaStreamWaitEvent(st, ev_panel, 0));
         KCU(cudaGetLastError());
         int info = 0, pert = 0;
         unsigned long long minr = inf_bits;
@@ -675,8 +1039,43 @@ struct BandLDLT {
         return SROM_OK;
     }
 
-    // X (n x nrhs, ldx, permuted order) <- K~^-1 X
-    int solve(double2 *X, int64_t ldx, int nrhs, Err &E) {
+    // Launch of a block step that may overlap the end of the launch before it (see wait_for_previous).
+    template <typename... P, typename... A>
+    cudaError_t chained(void (*kernel)(P...), int grid, size_t smem, A... args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(KT);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    }
+
+    // X (n x nrhs, ldx, permuted order) <- K~^-1 X; tmp: another n x nrhs (ldt)
+    int solve(double2 *X, int64_t ldx, int nrhs, double2 *tmp, int64_t ldt, Err &E) {
+        if (nrhs <= SOLVE_RMAX) {
+            for (int64_t j0 = 0; j0 < n; j0 += NB) {
+                const int nb = (int)std::min<int64_t>(NB, n - j0), rows = (int)std::min<int64_t>(bw, n - j0 - nb);
+                KCU(chained(solve_forward_kernel, std::max(1, (rows + NB - 1) / NB), forward_smem(nrhs), band, ldab, j0, nb,
+                            rows, X, ldx, tmp, ldt, nrhs));
+            }
+            for (int64_t j0 = ((n - 1) / NB) * NB; j0 >= 0; j0 -= NB) {
+                const int nb = (int)std::min<int64_t>(NB, n - j0), rows = (int)std::min<int64_t>(bw, n - j0 - nb);
+                int splits = 1;
+                int64_t kchunk = rows;
+                zgemm_split(nb, nrhs, rows, 1, sms, zwork_elems, &splits, &kchunk);
+                KCU(chained(solve_backward_kernel, splits, backward_smem(nrhs), band, ldab, j0, nb, rows, (int)kchunk, tmp, ldt,
+                            nrhs, zwork, d_ticket));
+            }
+            KCU(cudaMemcpy2DAsync(X, sizeof(double2) * ldx, tmp, sizeof(double2) * ldt, sizeof(double2) * n, nrhs,
+                                  cudaMemcpyDeviceToDevice, st));
+            KCU(cudaGetLastError());
+            return SROM_OK;
+        }
         const size_t smem = sizeof(double2) * NB * SLD;
         const int tgrid = (nrhs + KT / 32 - 1) / (KT / 32);
         for (int64_t j0 = 0; j0 < n; j0 += NB) {
@@ -835,6 +1234,18 @@ struct BandContext {
     double *d_nrm = nullptr;
     BandLDLT F;
 
+    BandContext() = default;
+    BandContext(const BandContext &) = delete;
+    BandContext &operator=(const BandContext &) = delete;
+    ~BandContext() {  // before the buffers go: the side stream uses them too
+        if (F.side) {
+            cudaStreamSynchronize(F.side);
+            cudaStreamDestroy(F.side);
+        }
+        if (F.ev_panel) cudaEventDestroy(F.ev_panel);
+        if (F.ev_rest) cudaEventDestroy(F.ev_rest);
+    }
+
     // The pattern's full symmetric form and RCM order: from the handle's cache when it holds
     // this pattern, else computed on the host and uploaded (into the cache when there is one).
     int init(cudaStream_t stream, int64_t n_rows, int64_t nnz, const int64_t *rowptr, const int *colind, int base,
@@ -868,7 +1279,7 @@ struct BandContext {
         F.n = n;
         F.bw = bw;
         F.ldab = bw + 2 * NB + 1;
-        F.ldw = (int)(2 * bw + NB);
+        F.ldw = (int)((bw + 7) / 8 * 8);
         F.st = st;
         auto need = [&](cudaError_t e, const char *what) {
             if (e != cudaSuccess)
@@ -878,8 +1289,9 @@ struct BandContext {
             return e == cudaSuccess;
         };
         if (!need(B.alloc(&F.band, (size_t)(n + 2 * NB) * F.ldab), "the band factor") ||
-            !need(B.alloc(&F.W, (size_t)F.ldw * NB), "the panel") ||
-            !need(B.alloc(&F.Lp, (size_t)F.ldw * NB), "the panel") || !need(B.alloc(&F.d_info, 1), "info"))
+            !need(B.alloc(&F.W, (size_t)2 * F.ldw * NB), "the panel") ||
+            !need(B.alloc(&F.Lp, (size_t)2 * F.ldw * NB), "the panel") || !need(B.alloc(&F.d_info, 1), "info") ||
+            !need(B.alloc(&F.d_ticket, 1), "info"))
             return E.code;
         if (reuse) {
             d_frp = cache->d_frp;
@@ -926,7 +1338,17 @@ struct BandContext {
             !need(B.alloc(&F.d_pert, 1), "the pivot statistics"))
             return E.code;
         const size_t smem = sizeof(double2) * NB * SLD;
-        KCU(cudaFuncSetAttribute(ldlt_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KCU(cudaFuncSetAttribute(ldlt_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UP_SMEM));
+        KCU(cudaFuncSetAttribute(solve_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)forward_smem(SOLVE_RMAX)));
+        KCU(cudaFuncSetAttribute(solve_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)backward_smem(SOLVE_RMAX)));
+        KCU(cudaMemsetAsync(F.d_ticket, 0, sizeof(unsigned), st));
+        int lo = 0, hi = 0;
+        KCU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+        KCU(cudaStreamCreateWithPriority(&F.side, cudaStreamNonBlocking, hi));
+        KCU(cudaEventCreateWithFlags(&F.ev_panel, cudaEventDisableTiming));
+        KCU(cudaEventCreateWithFlags(&F.ev_rest, cudaEventDisableTiming));
         KCU(cudaFuncSetAttribute(ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(smem + sizeof(double2) * NB)));
         KCU(cudaFuncSetAttribute(trsv_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -945,8 +1367,6 @@ struct BandContext {
                 cache->nfull = nfull;
             }
         }
-        KCU(cudaMemsetAsync(F.W, 0, sizeof(double2) * F.ldw * NB, st));
-        KCU(cudaMemsetAsync(F.Lp, 0, sizeof(double2) * F.ldw * NB, st));
         return SROM_OK;
     }
 
@@ -964,7 +1384,7 @@ struct BandContext {
     // Y (n x m, ldy) = A^-1 X (n x m, ldx) with the current factor; work: n x m scratch
     int solve(const double2 *X, int64_t ldx, double2 *Y, int64_t ldy, int m, double2 *work, Err &E) {
         permute_kernel<<<grid_for(n * m, KT), KT, 0, st>>>(n, m, d_iperm, X, ldx, work, n, 1);
-        int s = F.solve(work, n, m, E);
+        int s = F.solve(work, n, m, Y, ldy, E);  // Y holds the half-solved block meanwhile
         if (s) return s;
         permute_kernel<<<grid_for(n * m, KT), KT, 0, st>>>(n, m, d_iperm, work, n, Y, ldy, 0);
         KCU(cudaGetLastError());

@@ -252,6 +252,19 @@ int64_t zgemm_work_elems(int m, int n, int k, int batch, int sms) {
     return splits > 1 ? splits * batch * (int64_t)m * n : 0;
 }
 
+// split over k when the tiles alone cannot fill the GPU and the workspace allows it
+void zgemm_split(int m, int n, int k, int batch, int sms, int64_t work_elems, int *splits, int64_t *kchunk) {
+    const int64_t tiles = (int64_t)((m + ZG_BM - 1) / ZG_BM) * ((n + ZG_BN - 1) / ZG_BN) * batch;
+    *splits = 1;
+    if (work_elems > 0 && tiles < 2LL * sms && k >= 4 * 64) {
+        int64_t s = std::min<int64_t>((2LL * sms + tiles - 1) / tiles, k / 64);
+        s = std::min<int64_t>(s, work_elems / std::max<int64_t>(1, (int64_t)batch * m * n));
+        *splits = (int)std::max<int64_t>(1, std::min<int64_t>(s, 1024));
+    }
+    *kchunk = ((int64_t)k + *splits - 1) / *splits;
+    *kchunk = (*kchunk + ZG_BK - 1) / ZG_BK * ZG_BK;
+}
+
 cudaError_t zgemm(const Zgemm &z, cudaStream_t st) {
     if (z.m <= 0 || z.n <= 0 || z.batch <= 0) return cudaSuccess;
     if (z.opa < ZG_N || z.opa > ZG_C || z.opb < ZG_N || z.opb > ZG_C) return cudaErrorInvalidValue;
@@ -275,17 +288,9 @@ cudaError_t zgemm(const Zgemm &z, cudaStream_t st) {
     g.sc = z.sc;
     g.batch = z.batch;
     g.work = z.work;
-    // split over k when the tiles alone cannot fill the GPU and the workspace allows it
-    const int64_t tiles = (int64_t)((g.m + ZG_BM - 1) / ZG_BM) * ((g.n + ZG_BN - 1) / ZG_BN) * g.batch;
     int splits = 1;
-    if (z.work && z.work_elems > 0 && tiles < 2LL * z.sms && g.k >= 4 * 64) {
-        int64_t s = std::min<int64_t>((2LL * z.sms + tiles - 1) / tiles, g.k / 64);
-        s = std::min<int64_t>(s, z.work_elems / std::max<int64_t>(1, (int64_t)g.batch * g.m * g.n));
-        splits = (int)std::max<int64_t>(1, std::min<int64_t>(s, 1024));
-    }
+    zgemm_split(g.m, g.n, g.k, g.batch, z.sms, z.work ? z.work_elems : 0, &splits, &g.kchunk);
     g.splits = splits;
-    g.kchunk = ((int64_t)g.k + splits - 1) / splits;
-    g.kchunk = (g.kchunk + ZG_BK - 1) / ZG_BK * ZG_BK;
     if ((int64_t)g.batch * splits > 65535) return cudaErrorInvalidValue;
     dim3 grid((unsigned)((g.m + ZG_BM - 1) / ZG_BM), (unsigned)((g.n + ZG_BN - 1) / ZG_BN), (unsigned)(g.batch * splits));
     // eight warps of 32 x 16 when each CTA has few k stages (their prologue and epilogue then

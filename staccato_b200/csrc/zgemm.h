@@ -32,6 +32,8 @@ struct Zgemm {
 
 cudaError_t zgemm(const Zgemm &z, cudaStream_t st);
 int64_t zgemm_work_elems(int m, int n, int k, int batch, int sms);
+// The split over k that zgemm takes with that workspace: partial sums of kchunk terms each.
+void zgemm_split(int m, int n, int k, int batch, int sms, int64_t work_elems, int *splits, int64_t *kchunk);
 
 // out (device) = ||x||_2 over count complex entries, deterministic; work: znorm2_work_doubles()
 size_t znorm2_work_doubles();
