@@ -150,13 +150,15 @@ def solve_batched(handle: _capi.Handle, A, B, precision: int = _capi.SROM_FP64,
     info = torch.empty(count, dtype=torch.int32, device=dev)
     omega = torch.zeros(1, dtype=torch.float64, device=dev)
     zb = 16  # bytes per complex128
-    descs = []
-    for i in range(count):
-        descs.append(RomDesc(n=n, r=r, F=1, ldk=n, K=C.c_void_p(Acm.data_ptr() + i * n * n * zb), M=None, D=None,
-                             eta=0.0, rhs=C.c_void_p(Bcm.data_ptr() + i * n * r * zb), ldb=n,
-                             omega=C.c_void_p(omega.data_ptr()), X=C.c_void_p(X.data_ptr() + i * n * r * zb),
-                             info=C.c_void_p(info.data_ptr() + 4 * i), steps=None, berr=None, LU=None, ipiv=None))
-    arr = (RomDesc * max(count, 1))(*descs)
+    # the descriptors of all systems at once, as columns of one array: filling a ctypes structure a
+    # system took 1.5 ms for 1000 of them, more than the sweep
+    descs = np.zeros(max(count, 1), dtype=np.dtype(RomDesc))
+    i = np.arange(count, dtype=np.uint64)
+    for name, value in (("n", n), ("r", r), ("F", 1), ("ldk", n), ("ldb", n), ("omega", omega.data_ptr())):
+        descs[name] = value
+    for name, base, step in (("K", Acm, n * n * zb), ("rhs", Bcm, n * r * zb), ("X", X, n * r * zb), ("info", info, 4)):
+        descs[name][:count] = np.uint64(base.data_ptr()) + i * np.uint64(step)
+    arr = descs.ctypes.data_as(C.POINTER(RomDesc))
     o = opts(precision, max_refine, 0.0, flags)
     check(handle.ptr, _capi.lib().srom_sweep(handle.ptr, arr, count, C.byref(o)))
     torch.cuda.synchronize(dev)  # the staged copies above must outlive the kernels
