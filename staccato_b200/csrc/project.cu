@@ -135,6 +135,126 @@ __device__ __forceinline__ void spmm_rows(int64_t row, const int64_t *__restrict
             }
 }
 
+// Whether the rows r0 .. r0 + 2 have the same column list (a warp vote; the trip count is warp-uniform).
+__device__ __forceinline__ bool same_columns(int64_t r0, const int64_t *__restrict__ rowptr,
+                                             const int *__restrict__ colind, int base, int lane) {
+    const int64_t a0 = rowptr[r0], a1 = rowptr[r0 + 1], a2 = rowptr[r0 + 2], a3 = rowptr[r0 + 3];
+    const int64_t len = a1 - a0;
+    bool same = (a2 - a1) == len && (a3 - a2) == len;
+    for (int64_t t0 = 0; same && t0 < len; t0 += 32) {
+        const int64_t t = t0 + lane;
+        bool eq = true;
+        if (t < len) {
+            const int c0 = colind[a0 - base + t];
+            eq = c0 == colind[a1 - base + t] && c0 == colind[a2 - base + t];
+        }
+        same = __all_sync(0xffffffffu, eq);
+    }
+    return same;
+}
+
+// Two matrices of one pattern, up to 48 basis columns, on the FP64 tensor cores: the three rows of a node and the two matrices are
+// six of the eight rows of an m8n8k4 MMA whose k runs over four consecutive entries, and the gathered Vt rows
+// are its B operand.  A lane reads two neighbouring columns at once (16 bytes, eight lanes a 128-byte line) and
+// gives one to each of two MMAs, whose results for a lane are then four neighbouring columns.  With fused
+// multiply-adds every entry's six values were broadcast to the lanes from shared memory, which took twice the
+// arithmetic's time, and with fewer than 96 columns part of the lanes idle.  The gathers of 16 entries are in
+// flight together with the next 32 entries' columns and values.  An MMA adds its four products in order, so
+// the sums keep the order of the entries (Y's bits are those of spmm_rows); nodes whose rows differ in pattern
+// go through spmm_rows.  k and the row strides are even.  Bound by the gathers (a quarter-warp's 16-byte loads
+// fall in four lines).  Tet10 block: 0.20 -> 0.14 ms at k = 32, 0.22 -> 0.20 ms at k = 48.  One or three
+// matrices would fill three or nine rows of the eight: spmm_full_kernel.
+template <int TP>
+__global__ void __launch_bounds__(SPMM_THREADS, 2) spmm_mma_kernel(int64_t N, const int64_t *__restrict__ rowptr,
+                                                                   const int *__restrict__ colind, int base,
+                                                                   ProjVals vals, const double *__restrict__ Vt0, int k,
+                                                                   int ldv, double *__restrict__ Y0, int ldy,
+                                                                   int64_t y_stride) {
+    __shared__ SpmmStage stage[SPMM_WARPS];
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
+    SpmmStage &st = stage[threadIdx.x >> 5];
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int nwin = (k + 16 * TP - 1) / (16 * TP);
+    const int64_t nodes = (N + 2) / 3;
+    for (int64_t it = warp; it < nodes * nwin; it += nwarp) {
+        const int64_t r0 = it % nodes * 3;
+        const int w0 = (int)(it / nodes) * 16 * TP, kw = min(16 * TP, k - w0);
+        const double *Vt = Vt0 + w0;
+        double *Y = Y0 + w0;
+        const int nr = (int)min((int64_t)3, N - r0);
+        const int64_t p0 = rowptr[r0], p1 = rowptr[r0 + 1], p2 = rowptr[min(r0 + 2, N)], p3 = rowptr[min(r0 + 3, N)];
+        bool same = nr == 3 && p2 - p1 == p1 - p0 && p3 - p2 == p1 - p0;
+        const int len = (int)(p1 - p0);
+        if (same) {
+            // MMA row lr: matrix row lr / 2 of the node, matrix lr & 1 (rows 6 and 7: none)
+            const int rr = lr >> 1;
+            const double *va = (lr & 1 ? vals.v[1] : vals.v[0]) + (p0 - base) + (int64_t)min(rr, 2) * len;
+            const int *ci = colind + (p0 - base);
+            const int live_a = lr < 6 ? len : 0;
+            double acc[TP][2][2];
+#pragma unroll
+            for (int u = 0; u < TP; ++u) acc[u][0][0] = acc[u][0][1] = acc[u][1][0] = acc[u][1][1] = 0.0;
+            int col = 0, col1 = 0, col2 = 0;
+            double av[8];
+            auto fetch = [&](int c0) {  // columns of the three rows and this lane's values of 32 entries
+                const int e = min(c0 + lane, len - 1);
+                col = ci[e] - base;
+                col1 = ci[len + e] - base;
+                col2 = ci[2 * len + e] - base;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) av[g] = c0 + 4 * g + lk < live_a ? va[c0 + 4 * g + lk] : 0.0;
+            };
+            if (len > 0) fetch(0);
+            for (int c0 = 0; c0 < len; c0 += 32) {
+                same = __all_sync(0xffffffffu, col == col1 && col == col2);
+                if (!same) break;
+                const int mycol = col;
+                double a[8];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) a[g] = av[g];
+                if (c0 + 32 < len) fetch(c0 + 32);
+#pragma unroll
+                for (int h = 0; h < 8; h += 4) {
+                    if (c0 + 4 * h >= len) break;
+                    double2 v[4][TP];
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const int cg = __shfl_sync(0xffffffffu, mycol, 4 * (h + g) + lk);
+                        const double *vr = Vt + (int64_t)cg * ldv + 2 * lr;
+                        const bool live = c0 + 4 * (h + g) + lk < len;
+#pragma unroll
+                        for (int u = 0; u < TP; ++u)
+                            v[g][u] = live && 16 * u + 2 * lr < kw ? *reinterpret_cast<const double2 *>(vr + 16 * u)
+                                                                   : make_double2(0.0, 0.0);
+                    }
+#pragma unroll
+                    for (int g = 0; g < 4; ++g)
+#pragma unroll
+                        for (int u = 0; u < TP; ++u) {
+                            asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                                : "+d"(acc[u][0][0]), "+d"(acc[u][0][1]) : "d"(a[h + g]), "d"(v[g][u].x));
+                            asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                                : "+d"(acc[u][1][0]), "+d"(acc[u][1][1]) : "d"(a[h + g]), "d"(v[g][u].y));
+                        }
+                }
+            }
+            if (same && lr < 6) {
+                double *y = Y + (lr & 1) * y_stride + (r0 + rr) * ldy + 4 * lk;
+#pragma unroll
+                for (int u = 0; u < TP; ++u) {
+                    const int c = 16 * u + 4 * lk;
+                    if (c < kw) *reinterpret_cast<double2 *>(y + 16 * u) = make_double2(acc[u][0][0], acc[u][1][0]);
+                    if (c + 2 < kw) *reinterpret_cast<double2 *>(y + 16 * u + 2) = make_double2(acc[u][0][1], acc[u][1][1]);
+                }
+            }
+        }
+        if (!same)
+            for (int r = 0; r < nr; ++r)
+                spmm_rows<(TP + 1) / 2, 2, 1>(r0 + r, rowptr, colind, base, vals, Vt, kw, ldv, Y, ldy, y_stride, lane, st);
+    }
+}
+
 template <int CPL, int NMAT>
 __global__ void __launch_bounds__(SPMM_THREADS) spmm_full_kernel(int64_t N, const int64_t *__restrict__ rowptr,
                                                                  const int *__restrict__ colind, int base,
@@ -148,22 +268,7 @@ __global__ void __launch_bounds__(SPMM_THREADS) spmm_full_kernel(int64_t N, cons
     const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t r0 = warp * 3; r0 < N; r0 += nwarp * 3) {
         const int nr = (int)min((int64_t)3, N - r0);
-        bool same = nr == 3;
-        if (same) {
-            const int64_t a0 = rowptr[r0], a1 = rowptr[r0 + 1], a2 = rowptr[r0 + 2], a3 = rowptr[r0 + 3];
-            const int64_t len = a1 - a0;
-            same = (a2 - a1) == len && (a3 - a2) == len;
-            // the trip count is warp-uniform, so every lane takes part in every vote
-            for (int64_t t0 = 0; same && t0 < len; t0 += 32) {
-                const int64_t t = t0 + lane;
-                bool eq = true;
-                if (t < len) {
-                    const int c0 = colind[a0 - base + t];
-                    eq = c0 == colind[a1 - base + t] && c0 == colind[a2 - base + t];
-                }
-                same = __all_sync(0xffffffffu, eq);
-            }
-        }
+        const bool same = nr == 3 && same_columns(r0, rowptr, colind, base, lane);
         if (same) {
             spmm_rows<CPL, NMAT, 3>(r0, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride, lane, st);
         } else {
@@ -186,6 +291,14 @@ static void spmm_full_launch(int grid, cudaStream_t st, int64_t N, const int64_t
         grid = std::min(grid, per_sm * sms);
     spmm_full_kernel<CPL, NMAT><<<grid, SPMM_THREADS, 0, st>>>(N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy,
                                                                y_stride);
+}
+
+template <int TP>
+static void spmm_mma_launch(int grid, cudaStream_t st, int64_t N, const int64_t *rowptr, const int *colind, int base,
+                            const ProjVals &vals, const double *Vt, int k, int ldv, double *Y, int ldy, int64_t y_stride,
+                            int sms) {
+    spmm_mma_kernel<TP><<<std::min(grid, 2 * sms), SPMM_THREADS, 0, st>>>(N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy,
+                                                                         y_stride);
 }
 
 template <int CPL>
@@ -222,8 +335,8 @@ __global__ void spmm_upper_mirror_kernel(int64_t N, const int64_t *__restrict__ 
 
 // ---- R_m partial = Vt[rows]^T Y_m[rows] on FP64 tensor cores ------------------------------
 // One launch covers nm matrices and one window of R: ka rows (basis columns of Vt, row stride
-// ldv) by kb columns (columns of Y_m, row stride ldy), both <= 128.  Warp w owns matrix
-// w / nband and the 8-row band w % nband of the window (nband = kap / 8), 8x8 tiles across it.
+// ldv) by kb columns (columns of Y_m, row stride ldy), both <= 128.  The warps share
+// out the matrices and the 8 x 8 tiles of the window.
 // The rows of Vt and of the nm Y's are staged 32 at a time in shared memory (leading
 // dimension padded by 4 keeps the fragment loads free of bank conflicts); the Vt chunk is
 // staged once for all nm matrices, and the chunks are double-buffered with cp.async so the
@@ -242,49 +355,56 @@ struct VtyWindow {
     int64_t y_stride;  // between matrices
 };
 
-template <int TMAX, int MAXT>
+// A warp's share is two 8-row bands by half of the tiles across: eight fragment reads for twelve MMAs (one
+// band by all tiles took thirteen, and the shared-memory datapath as long as the MMAs).  PAIRS: rows of even
+// length, copied 16 bytes at a time, a warp a row.
+template <int TH, int MAXT, bool PAIRS>
 __global__ void __launch_bounds__(MAXT) vty_partial_kernel(int64_t N, VtyWindow w, int nm, int64_t chunks_per_cta,
                                                            double *__restrict__ partial) {
-    extern __shared__ double sh[];
+    extern __shared__ __align__(16) double sh[];
     const int kap = (w.ka + 7) & ~7, kbp = (w.kb + 7) & ~7;
     const int lda = kap + 4, ldb = kbp + 4;
-    const int nband = kap / 8, ntile = kbp / 8;
+    const int nband = kap / 8, ntile = kbp / 8, nbp = (nband + 1) / 2, th = (ntile + 1) / 2;
     const int a_sz = 32 * lda, b_sz = 32 * ldb;
     const int stage = a_sz + nm * b_sz;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int mloc = warp / nband, band = warp % nband;
-    const bool active = mloc < nm;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int mloc = warp / (2 * nbp), band0 = warp % (2 * nbp) / 2 * 2, t0 = (warp & 1) * th;
+    const bool second = band0 + 1 < nband;
+    const int nt = min(th, ntile - t0);
     const int64_t n_chunks = (N + 31) / 32;
     const int64_t c_begin = (int64_t)blockIdx.x * chunks_per_cta;
     const int64_t c_end = min(n_chunks, c_begin + chunks_per_cta);
-    const int a_tot = 32 * kap, total = a_tot + nm * 32 * kbp;
 
     auto issue = [&](int64_t ch, int buf) {
         double *dst0 = sh + buf * stage;
         const int64_t r0 = ch * 32;
         const int nr = (int)min((int64_t)32, N - r0);
-        for (int e = threadIdx.x; e < total; e += blockDim.x) {
-            double *dst;
-            const double *src = nullptr;
-            if (e < a_tot) {
-                const int rr = e / kap, c = e - rr * kap;
-                dst = dst0 + rr * lda + c;
-                if (rr < nr && c < w.ka) src = w.Vt + (r0 + rr) * w.ldv + c;
-            } else {
-                const int eb = e - a_tot, mat = eb / (32 * kbp), rem = eb - mat * 32 * kbp;
-                const int rr = rem / kbp, c = rem - rr * kbp;
-                dst = dst0 + a_sz + mat * b_sz + rr * ldb + c;
-                if (rr < nr && c < w.kb) src = w.Y + mat * w.y_stride + (r0 + rr) * w.ldy + c;
+        for (int row = warp; row < 32 * (1 + nm); row += nw) {
+            const int rr = row & 31, which = row >> 5;  // 0: Vt, else matrix which - 1
+            const bool isa = which == 0;
+            const int kk = isa ? w.ka : w.kb, kp = isa ? kap : kbp;
+            double *dst = dst0 + (isa ? rr * lda : a_sz + (which - 1) * b_sz + rr * ldb);
+            const double *src = isa ? w.Vt + (r0 + rr) * w.ldv : w.Y + (which - 1) * w.y_stride + (r0 + rr) * w.ldy;
+            constexpr int PER = PAIRS ? 2 : 1;
+            for (int c = PER * lane; c < kp; c += 32 * PER) {
+                const unsigned d = (unsigned)__cvta_generic_to_shared(dst + c);
+                if (rr < nr && c < kk) {
+                    if constexpr (PAIRS) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + c));
+                    else cp_async8(dst + c, src + c);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < PER; ++h) dst[c + h] = 0.0;
+                }
             }
-            if (src) cp_async8(dst, src);
-            else *dst = 0.0;
         }
         asm volatile("cp.async.commit_group;");
     };
 
-    double acc[TMAX][2];
+    double acc[2][TH][2];
 #pragma unroll
-    for (int t = 0; t < TMAX; ++t) acc[t][0] = acc[t][1] = 0.0;
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int t = 0; t < TH; ++t) acc[x][t][0] = acc[x][t][1] = 0.0;
     if (c_begin < c_end) issue(c_begin, 0);
     for (int64_t ch = c_begin; ch < c_end; ++ch) {
         const int buf = (int)((ch - c_begin) & 1);
@@ -295,53 +415,78 @@ __global__ void __launch_bounds__(MAXT) vty_partial_kernel(int64_t N, VtyWindow 
             asm volatile("cp.async.wait_group 0;");
         }
         __syncthreads();
-        if (active) {
-            const double *sV = sh + buf * stage;
-            const double *sY = sV + a_sz + mloc * b_sz;
+        {
+            const double *sV = sh + buf * stage + 8 * band0 + (lane >> 2);
+            const double *sY = sh + buf * stage + a_sz + mloc * b_sz + 8 * t0 + (lane >> 2);
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
                 const int rr = 4 * kk + (lane & 3);
-                const double a = sV[rr * lda + 8 * band + (lane >> 2)];
+                const double a0 = sV[rr * lda], a1 = second ? sV[rr * lda + 8] : 0.0;
 #pragma unroll
-                for (int t = 0; t < TMAX; ++t) {
-                    if (t < ntile) {
-                        const double b = sY[rr * ldb + 8 * t + (lane >> 2)];
+                for (int t = 0; t < TH; ++t) {
+                    if (t < nt) {
+                        const double b = sY[rr * ldb + 8 * t];
                         asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                                     : "+d"(acc[t][0]), "+d"(acc[t][1])
-                                     : "d"(a), "d"(b));
+                                     : "+d"(acc[0][t][0]), "+d"(acc[0][t][1])
+                                     : "d"(a0), "d"(b));
+                        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                                     : "+d"(acc[1][t][0]), "+d"(acc[1][t][1])
+                                     : "d"(a1), "d"(b));
                     }
                 }
             }
         }
         __syncthreads();
     }
-    if (active) {
-        // lane holds D[row = lane/4][col = 2*(lane%4) + {0,1}] of tile (band, t)
-        const int ra = 8 * band + (lane >> 2);
-        double *P = partial + ((int64_t)mloc * gridDim.x + blockIdx.x) * kap * kbp;
+    // lane holds D[row = lane/4][col = 2*(lane%4) + {0,1}] of tile (band, t)
+    double *P = partial + ((int64_t)mloc * gridDim.x + blockIdx.x) * kap * kbp;
 #pragma unroll
-        for (int t = 0; t < TMAX; ++t) {
-            if (t < ntile) {
-                const int cb = 8 * t + 2 * (lane & 3);
-                P[ra + (int64_t)cb * kap] = acc[t][0];
-                P[ra + (int64_t)(cb + 1) * kap] = acc[t][1];
+    for (int x = 0; x < 2; ++x) {
+        if (x == 1 && !second) break;
+        const int ra = 8 * (band0 + x) + (lane >> 2);
+#pragma unroll
+        for (int t = 0; t < TH; ++t) {
+            if (t < nt) {
+                const int cb = 8 * (t0 + t) + 2 * (lane & 3);
+                P[ra + (int64_t)cb * kap] = acc[x][t][0];
+                P[ra + (int64_t)(cb + 1) * kap] = acc[x][t][1];
             }
         }
     }
 }
 
-// out.r[m][a + b * ldr] = sum over the CTA partials, in CTA order (deterministic)
+// Sum of part[blk * stride] over the CTA partials, by RED_SEG threads an element (threadIdx.y): segment y
+// takes blk = y, y + RED_SEG, ..., and the segments are added in order (deterministic).  With one thread an
+// element the few thousand elements of a small result left the GPU idle on one chain of nblk loads
+// (43 us for two 96 x 96 results of 148 partials, 59 us for a Gram-Schmidt panel).  Valid in segment 0.
+constexpr int RED_SEG = 16;
+__device__ __forceinline__ double sum_partials(const double *__restrict__ part, int nblk, int64_t stride, bool live) {
+    __shared__ double red[RED_SEG][33];
+    double s = 0.0;
+    if (live) {
+#pragma unroll 5
+        for (int blk = threadIdx.y; blk < nblk; blk += RED_SEG) s += part[(int64_t)blk * stride];
+    }
+    red[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    s = 0.0;
+    if (threadIdx.y == 0) {
+#pragma unroll
+        for (int y = 0; y < RED_SEG; ++y) s += red[y][threadIdx.x];
+    }
+    return s;
+}
+
+// out.r[m][a + b * ldr] = sum over the CTA partials
 __global__ void reduce_partials_kernel(const double *__restrict__ partial, int nblk, int nmat, int ka, int kb,
                                        int kap, int kbp, ProjOut out, int ldr) {
-    const int64_t tot = (int64_t)nmat * ka * kb;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-        const int m = (int)(e / ((int64_t)ka * kb));
-        const int rem = (int)(e % ((int64_t)ka * kb));
-        const int a = rem % ka, b = rem / ka;
-        double s = 0.0;
-        for (int blk = 0; blk < nblk; ++blk) s += partial[((int64_t)m * nblk + blk) * kap * kbp + a + (int64_t)b * kap];
-        out.r[m][a + (int64_t)b * ldr] = s;
-    }
+    const int64_t e = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    const bool live = e < (int64_t)nmat * ka * kb;
+    const int m = live ? (int)(e / ((int64_t)ka * kb)) : 0;
+    const int rem = live ? (int)(e % ((int64_t)ka * kb)) : 0;
+    const int a = rem % ka, b = rem / ka;
+    const double s = sum_partials(partial + (int64_t)m * nblk * kap * kbp + a + (int64_t)b * kap, nblk, (int64_t)kap * kbp, live);
+    if (live && threadIdx.y == 0) out.r[m][a + (int64_t)b * ldr] = s;
 }
 
 // ---- block Gram-Schmidt with re-orthogonalisation --------------------------------------
@@ -361,36 +506,51 @@ constexpr int GS_THREADS = 512;
 constexpr int GS_HCHUNK = 128;  // rows of H staged per round of the row update
 
 // part[blk][x0 + i][c] = sum over this CTA's rows of V[r, x0 + i] * V[r, j0 + c]
-// (i < w, c < b), on the FP64 tensor cores; chunks of 32 rows double-buffered with cp.async.
+// (i < w, c < b), on the FP64 tensor cores; chunks of 32 rows through a ring of GS_STAGES cp.async
+// stages (one CTA an SM: with two stages too little was in flight to reach the L2's rate).  PAIRS: V and ldv
+// allow 16-byte copies of two rows.  The panel is staged once where the window ends with it.
+constexpr int GS_STAGES = 4;
+template <bool PAIRS>
 __global__ void __launch_bounds__(GS_THREADS) gs_gram_kernel(const double *__restrict__ V, int64_t N, int64_t ldv,
                                                              int x0, int w, int j0, int b, int rows_c,
                                                              int64_t chunks_per_cta, double *__restrict__ part) {
-    extern __shared__ double sh[];
+    extern __shared__ __align__(16) double sh[];
     const int wp = (w + 7) & ~7, bp = (b + 7) & ~7;
-    const int stage = (wp + bp) * GS_LDR;
+    const bool own = x0 + w == j0 + b && w >= b;  // the window's last columns are the panel
+    const int po = own ? w - b : wp;              // staged column of the panel's first
+    const int cols = own ? po + bp : wp + bp;     // wp <= cols, as w = po + b
+    const int stage = (GS_WIN + GS_B) * GS_LDR;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nband = wp / 8, ntile = bp / 8;
     const int64_t n_chunks = (N + 31) / 32;
     const int64_t c_begin = (int64_t)blockIdx.x * chunks_per_cta;
     const int64_t c_end = min(n_chunks, c_begin + chunks_per_cta);
-    const int total = (wp + bp) * 32;
 
-    auto issue = [&](int64_t ch, int buf) {
-        double *dst0 = sh + buf * stage;
-        const int64_t r0 = ch * 32;
-        const int nr = (int)min((int64_t)32, N - r0);
-        for (int e = threadIdx.x; e < total; e += blockDim.x) {
-            const int col = e >> 5, rr = e & 31;  // staged column col: X for col < wp, P after
-            const bool isx = col < wp;
-            const int cc = isx ? col : col - wp;
-            const bool ok = rr < nr && (isx ? cc < w : cc < b);
-            double *dst = dst0 + col * GS_LDR + rr;
-            if (ok) {
-                const int64_t vc = isx ? x0 + cc : j0 + cc;
+    auto issue = [&](int64_t ch) {
+        if (ch < c_end) {
+            double *dst0 = sh + (int)((ch - c_begin) % GS_STAGES) * stage;
+            const int64_t r0 = ch * 32;
+            const int nr = (int)min((int64_t)32, N - r0);
+            constexpr int LPC = PAIRS ? 16 : 32;  // lanes a column
+            for (int col = threadIdx.x / LPC; col < cols; col += GS_THREADS / LPC) {
+                const int rr = (threadIdx.x % LPC) * (32 / LPC);
+                const bool isp = col >= po;
+                const int cc = isp ? col - po : col;
+                const bool ok = isp ? cc < b : cc < w;
+                double *dst = dst0 + col * GS_LDR + rr;
+                const double *src = V + r0 + rr + (int64_t)(isp ? j0 + cc : x0 + cc) * ldv;
                 const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(V + r0 + rr + vc * ldv));
-            } else {
-                *dst = 0.0;
+                if (PAIRS && ok && rr + 1 < nr) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 32 / LPC; ++h) {
+                        if (ok && rr + h < nr)
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d + 8 * h), "l"(src + h));
+                        else
+                            dst[h] = 0.0;
+                    }
+                }
             }
         }
         asm volatile("cp.async.commit_group;");
@@ -399,19 +559,15 @@ __global__ void __launch_bounds__(GS_THREADS) gs_gram_kernel(const double *__res
     double acc[4][2];
 #pragma unroll
     for (int t = 0; t < 4; ++t) acc[t][0] = acc[t][1] = 0.0;
-    if (c_begin < c_end) issue(c_begin, 0);
+    for (int q = 0; q < GS_STAGES - 1; ++q) issue(c_begin + q);
     for (int64_t ch = c_begin; ch < c_end; ++ch) {
-        const int buf = (int)((ch - c_begin) & 1);
-        if (ch + 1 < c_end) {
-            issue(ch + 1, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;");
-        } else {
-            asm volatile("cp.async.wait_group 0;");
-        }
-        __syncthreads();
+        const int buf = (int)((ch - c_begin) % GS_STAGES);
+        asm volatile("cp.async.wait_group %0;" ::"n"(GS_STAGES - 2));
+        __syncthreads();  // the chunk is in; everyone is done with the one before, whose place the next takes
+        issue(ch + GS_STAGES - 1);
         if (warp < nband) {
             const double *sX = sh + buf * stage;
-            const double *sP = sX + wp * GS_LDR;
+            const double *sP = sX + po * GS_LDR;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {
                 const int rr = 4 * kk + (lane & 3);
@@ -427,8 +583,8 @@ __global__ void __launch_bounds__(GS_THREADS) gs_gram_kernel(const double *__res
                 }
             }
         }
-        __syncthreads();
     }
+    asm volatile("cp.async.wait_group 0;");
     if (warp < nband) {
         const int i = x0 + 8 * warp + (lane >> 2);
         double *P = part + (int64_t)blockIdx.x * rows_c * GS_B;
@@ -443,124 +599,163 @@ __global__ void __launch_bounds__(GS_THREADS) gs_gram_kernel(const double *__res
     }
 }
 
-// C[i][c] = sum_blk part[blk][i][c] in CTA order (deterministic)
+// C[i][c] = sum_blk part[blk][i][c]
 __global__ void gs_reduce_kernel(const double *__restrict__ part, int nblk, int rows_c, double *__restrict__ Cm) {
-    const int64_t tot = (int64_t)rows_c * GS_B;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int blk = 0; blk < nblk; ++blk) s += part[(int64_t)blk * tot + e];
-        Cm[e] = s;
-    }
+    const int64_t tot = (int64_t)rows_c * GS_B, e = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    const double s = sum_partials(part + e, nblk, tot, e < tot);
+    if (e < tot && threadIdx.y == 0) Cm[e] = s;
 }
 
-// One CTA: G' = G - H^T H, Cholesky R^T R = G', Rinv = R^-1 (upper), written to rinv[a][c].
-__global__ void gs_chol_kernel(const double *__restrict__ Cm, int j0, int b, double *__restrict__ rinv) {
+// One CTA: G' = G - H^T H, Cholesky R^T R = G', Rinv = R^-1 (upper), written to rinv[a][c].  Thread (a, c)
+// holds rows a, a + 8, a + 16, a + 24 of column c.  The elimination multiplies by the pivot's reciprocal (one
+// a step, 31 dependent steps) and the rows are scaled by 1 / sqrt(pivot) at the end; Rinv's columns take a lane
+// each, right-looking, in registers.
+constexpr int GS_CT = 256, GS_CR = GS_B * GS_B / GS_CT;
+__global__ void __launch_bounds__(GS_CT) gs_chol_kernel(const double *__restrict__ Cm, int j0, int b,
+                                                        double *__restrict__ rinv) {
     __shared__ double G[GS_B][GS_B + 1];
-    __shared__ double R[GS_B][GS_B + 1];
-    for (int e = threadIdx.x; e < GS_B * GS_B; e += blockDim.x) {
-        const int a = e / GS_B, c = e % GS_B;
-        double g = 0.0;
-        if (a < b && c < b) {
-            g = Cm[(int64_t)(j0 + a) * GS_B + c];
-            double s = 0.0;
-            for (int i = 0; i < j0; ++i) s = fma(Cm[(int64_t)i * GS_B + a], Cm[(int64_t)i * GS_B + c], s);
-            g -= s;
-        }
-        G[a][c] = g;
-        R[a][c] = 0.0;
+    __shared__ double rd[GS_B];  // 1 / R[j][j]
+    const int a0 = threadIdx.x / GS_B, c = threadIdx.x % GS_B;
+    double g[GS_CR];
+#pragma unroll
+    for (int q = 0; q < GS_CR; ++q) g[q] = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < j0; ++i) {
+        const double hc = Cm[(int64_t)i * GS_B + c];
+#pragma unroll
+        for (int q = 0; q < GS_CR; ++q) g[q] = fma(Cm[(int64_t)i * GS_B + a0 + 8 * q], hc, g[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < GS_CR; ++q) {
+        const int a = a0 + 8 * q;
+        // unit diagonal past a short panel
+        g[q] = a < b && c < b ? Cm[(int64_t)(j0 + a) * GS_B + c] - g[q] : (a == c ? 1.0 : 0.0);
+        G[a][c] = g[q];
     }
     __syncthreads();
-    // right-looking Cholesky of the symmetric G' (upper factor R, row by row)
-    for (int j = 0; j < b; ++j) {
-        const double d = sqrt(G[j][j]);
-        __syncthreads();
-        for (int c = j + threadIdx.x; c < b; c += blockDim.x) R[j][c] = c == j ? d : G[j][c] / d;
-        __syncthreads();
-        for (int e = threadIdx.x; e < (b - j - 1) * (b - j - 1); e += blockDim.x) {
-            const int a = j + 1 + e / (b - j - 1), c = j + 1 + e % (b - j - 1);
-            G[a][c] = fma(-R[j][a], R[j][c], G[a][c]);
+    // G = L D L^T by rows: row j is final before step j, and R[j][c] = G[j][c] / sqrt(G[j][j])
+    for (int j = 0; j + 1 < b; ++j) {
+        const double t = G[j][c] * __drcp_rn(G[j][j]);
+#pragma unroll
+        for (int q = 0; q < GS_CR; ++q) {
+            const int a = a0 + 8 * q;
+            if (a > j && c > j) {
+                g[q] = fma(-G[j][a], t, g[q]);
+                G[a][c] = g[q];  // read only as row a of a later step
+            }
         }
         __syncthreads();
     }
-    // Rinv column c by back substitution: R x = e_c, one thread per column
-    for (int c = threadIdx.x; c < GS_B; c += blockDim.x) {
+    if (a0 == 0) rd[c] = 1.0 / sqrt(G[c][c]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < GS_CR; ++q) {
+        const int a = a0 + 8 * q;
+        if (a < c) G[a][c] = g[q] * rd[a];
+    }
+    __syncthreads();
+    if (threadIdx.x < GS_B) {
+        // column c of R^-1: x_i = (e_c - sum_{l > i} R[i][l] x_l) / R[i][i] from the last row
         double x[GS_B];
 #pragma unroll
-        for (int i = 0; i < GS_B; ++i) x[i] = 0.0;
-        if (c < b) {
-            for (int i = c; i >= 0; --i) {
-                double s = i == c ? 1.0 : 0.0;
-                for (int l = i + 1; l <= c; ++l) s = fma(-R[i][l], x[l], s);
-                x[i] = s / R[i][i];
-            }
+        for (int i = 0; i < GS_B; ++i) x[i] = i == c && c < b ? 1.0 : 0.0;
+#pragma unroll
+        for (int l = GS_B - 1; l >= 0; --l) {
+            x[l] *= rd[l];
+#pragma unroll
+            for (int i = 0; i < l; ++i) x[i] = fma(-G[i][l], x[l], x[i]);
         }
-        for (int i = 0; i < GS_B; ++i) rinv[i * GS_B + c] = x[i];
+#pragma unroll
+        for (int i = 0; i < GS_B; ++i) rinv[i * GS_B + c] = i <= c ? x[i] : 0.0;
     }
 }
 
-// Two threads per row, 16 panel columns each: p <- (p - q H) Rinv with q = V[r, :j0] and
-// p = V[r, j0:j0+b].  Lane l of a warp takes row (l & 15) and columns 16 (l >> 4) ...; the
-// upper half reads the lower half's p through shuffles for the triangular product.
-constexpr int GS_HALF = GS_B / 2;
-__global__ void __launch_bounds__(256, 2) gs_update_kernel(double *__restrict__ V, int64_t N, int64_t ldv, int j0, int b,
+// p <- (p - q H) Rinv with q = V[r, :j0] and p = V[r, j0:j0+b]: 16 rows a warp, both products on the FP64
+// tensor cores (H from shared memory, the rows of V straight from global memory in fragment order, p - q H
+// through shared memory into the second product's A operand).  HBM / L2 bound; as fused multiply-adds with H
+// broadcast from shared memory every row cost eight 16-byte reads for 16 multiply-adds.
+constexpr int GS_UW = 8;             // warps of a CTA, 16 rows each
+constexpr int GS_LDB = GS_B + 4;     // 4 modulo 16 doubles: conflict-free fragments
+__device__ __forceinline__ void gs_dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+__global__ void __launch_bounds__(32 * GS_UW, 3) gs_update_kernel(double *__restrict__ V, int64_t N, int64_t ldv, int j0, int b,
                                                         const double *__restrict__ Cm, const double *__restrict__ rinv) {
-    __shared__ __align__(16) double Hs[GS_HCHUNK * GS_B];
-    __shared__ __align__(16) double Rs[GS_B * GS_B];
-    for (int e = threadIdx.x; e < GS_B * GS_B; e += blockDim.x) Rs[e] = rinv[e];
-    const int lane = threadIdx.x & 31, half = lane >> 4;
-    const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane) / 2 + (lane & 15);
-    const bool live = r < N;
-    const int cb = half * GS_HALF;
-    double p[GS_HALF];
+    __shared__ double Hs[GS_HCHUNK * GS_LDB];  // rows of H; later the warps' p - q H
+    __shared__ double Rs[GS_B * GS_LDB];
+    static_assert(GS_UW * 16 <= GS_HCHUNK, "the warps' rows fit the place of H");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lk = lane & 3;
+    for (int e = threadIdx.x; e < GS_B * GS_B; e += blockDim.x) Rs[e / GS_B * GS_LDB + e % GS_B] = rinv[e];
+    const int64_t r0 = ((int64_t)blockIdx.x * GS_UW + warp) * 16;
+    double acc[2][4][2];
 #pragma unroll
-    for (int c = 0; c < GS_HALF; ++c) p[c] = (live && cb + c < b) ? V[r + (int64_t)(j0 + cb + c) * ldv] : 0.0;
-    for (int i0 = 0; i0 < j0; i0 += GS_HCHUNK) {
-        const int ni = min(GS_HCHUNK, j0 - i0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < ni * GS_B; e += blockDim.x) Hs[e] = Cm[(int64_t)i0 * GS_B + e];
-        __syncthreads();
-        if (live) {
-#pragma unroll 4
-            for (int i = 0; i < ni; ++i) {
-                const double q = V[r + (int64_t)(i0 + i) * ldv];
-                const double2 *h2 = reinterpret_cast<const double2 *>(Hs + i * GS_B + cb);
+    for (int x = 0; x < 2; ++x)
 #pragma unroll
-                for (int c2 = 0; c2 < GS_HALF / 2; ++c2) {
-                    const double2 hv = h2[c2];
-                    p[2 * c2] = fma(-q, hv.x, p[2 * c2]);
-                    p[2 * c2 + 1] = fma(-q, hv.y, p[2 * c2 + 1]);
-                }
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int64_t r = r0 + 8 * x + lr;
+                const int c = 8 * t + 2 * lk + h;
+                acc[x][t][h] = (r < N && c < b) ? V[r + (int64_t)(j0 + c) * ldv] : 0.0;
             }
+    for (int i0 = 0; i0 < j0; i0 += GS_HCHUNK) {
+        const int ni = min(GS_HCHUNK, j0 - i0);  // a multiple of GS_B
+        __syncthreads();
+        for (int e = threadIdx.x; e < ni * GS_B; e += blockDim.x)
+            Hs[e / GS_B * GS_LDB + e % GS_B] = Cm[(int64_t)i0 * GS_B + e];
+        __syncthreads();
+#pragma unroll 4
+        for (int i = 0; i < ni; i += 4) {
+            double q[2], h[4];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int64_t r = r0 + 8 * x + lr;
+                q[x] = r < N ? -V[r + (int64_t)(i0 + i + lk) * ldv] : 0.0;
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) h[t] = Hs[(i + lk) * GS_LDB + 8 * t + lr];
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int t = 0; t < 4; ++t) gs_dmma(acc[x][t], q[x], h[t]);
         }
     }
     __syncthreads();
-    // p <- p Rinv (upper): column c takes the row's p[0..c]
-    double o[GS_HALF];
+    double *T = Hs + warp * 16 * GS_LDB;
 #pragma unroll
-    for (int u = 0; u < GS_HALF; ++u) o[u] = 0.0;
+    for (int x = 0; x < 2; ++x)
 #pragma unroll
-    for (int i = 0; i < GS_HALF; ++i) {
-        const double lo = __shfl_sync(0xffffffffu, p[i], lane & 15);  // the row's p[i], i < 16
+        for (int t = 0; t < 4; ++t)
 #pragma unroll
-        for (int u = 0; u < GS_HALF; ++u) {
-            if (half == 0) {
-                if (i <= u) o[u] = fma(lo, Rs[i * GS_B + u], o[u]);
-            } else {
-                o[u] = fma(lo, Rs[i * GS_B + GS_HALF + u], o[u]);
+            for (int h = 0; h < 2; ++h) {
+                T[(8 * x + lr) * GS_LDB + 8 * t + 2 * lk + h] = acc[x][t][h];
+                acc[x][t][h] = 0.0;
             }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < GS_B; k += 4) {
+        double p[2];
+#pragma unroll
+        for (int x = 0; x < 2; ++x) p[x] = T[(8 * x + lr) * GS_LDB + k + lk];
+#pragma unroll
+        for (int t = k / 8; t < 4; ++t) {  // Rinv is upper triangular
+            const double rv = Rs[(k + lk) * GS_LDB + 8 * t + lr];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) gs_dmma(acc[x][t], p[x], rv);
         }
     }
-    if (half == 1) {
 #pragma unroll
-        for (int i = 0; i < GS_HALF; ++i)
+    for (int x = 0; x < 2; ++x)
 #pragma unroll
-            for (int u = 0; u < GS_HALF; ++u)
-                if (i <= u) o[u] = fma(p[i], Rs[(GS_HALF + i) * GS_B + GS_HALF + u], o[u]);
-    }
-    if (!live) return;
+        for (int t = 0; t < 4; ++t)
 #pragma unroll
-    for (int c = 0; c < GS_HALF; ++c)
-        if (cb + c < b) V[r + (int64_t)(j0 + cb + c) * ldv] = o[c];
+            for (int h = 0; h < 2; ++h) {
+                const int64_t r = r0 + 8 * x + lr;
+                const int c = 8 * t + 2 * lk + h;
+                if (r < N && c < b) V[r + (int64_t)(j0 + c) * ldv] = acc[x][t][h];
+            }
 }
 
 // ---- complex projection R = Z^H A V through the real kernels ------------------------------
@@ -669,7 +864,13 @@ cudaError_t launch_spmm(int64_t N, const int64_t *rowptr, const int *colind, int
         const int kw = std::min(PRJ_WIN, k - j0);
         const double *Vw = Vt + j0;
         double *Yw = Y + j0;
-        if (kw <= 32) launch_spmm_full<1>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
+        // two matrices, even rows (the window starts on a multiple of 128 columns), up to 48 columns: the tensor
+        // cores.  Beyond, a node's gathers no longer fit one warp's registers and its values and columns are read
+        // once a 48-column part (Tet10 block: 0.20 against 0.22 ms at 48 columns, 0.26 against 0.22 at 64)
+        if (n_mats == 2 && kw <= 48 && (k & 1) == 0 && (y_stride & 1) == 0) {
+            auto go = kw <= 32 ? spmm_mma_launch<2> : spmm_mma_launch<3>;
+            go(grid, st, N, rowptr, colind, base, vals, Vw, kw, k, Yw, k, y_stride, sms);
+        } else if (kw <= 32) launch_spmm_full<1>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
         else if (kw <= 64) launch_spmm_full<2>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
         else if (kw <= 96) launch_spmm_full<3>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
         else launch_spmm_full<4>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
@@ -696,12 +897,15 @@ size_t vty_partial_doubles(int k, int n_mats, int nblk) {
     return (size_t)nblk * n_mats * kp * kp;
 }
 
-template <int TMAX, int MAXT>
+template <int TH, int MAXT>
 static cudaError_t vty_launch(int64_t N, const VtyWindow &w, int nm, int nblk, double *partial, cudaStream_t st) {
     const int kap = (w.ka + 7) & ~7, kbp = (w.kb + 7) & ~7;
-    const int threads = 32 * nm * (kap / 8);
+    const int threads = 32 * nm * 2 * ((kap / 8 + 1) / 2);
     const size_t smem = sizeof(double) * (size_t)2 * 32 * ((kap + 4) + (size_t)nm * (kbp + 4));
-    auto kf = vty_partial_kernel<TMAX, MAXT>;
+    // rows of even length: every row of Vt and Y starts on 16 bytes
+    const bool pairs = ((w.ldv | w.ldy | w.ka | w.kb) & 1) == 0 && (w.y_stride & 1) == 0 &&
+                       ((reinterpret_cast<uintptr_t>(w.Vt) | reinterpret_cast<uintptr_t>(w.Y)) & 15) == 0;
+    auto kf = pairs ? vty_partial_kernel<TH, MAXT, true> : vty_partial_kernel<TH, MAXT, false>;
     cudaError_t e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t n_chunks = (N + 31) / 32;
@@ -726,17 +930,17 @@ cudaError_t launch_vty(int64_t N, int k, const double *Vt, const double *Y, int6
                 const VtyWindow w{Vt + i0, ka, k, Y + m0 * y_stride + j0, kb, k, y_stride};
                 double *Pm = partial + (int64_t)m0 * nblk * kap * kbp;
                 cudaError_t e;
-                if (ntile <= 4) e = vty_launch<4, 768>(N, w, nm, nblk, Pm, st);
-                else if (ntile <= 8) e = vty_launch<8, 768>(N, w, nm, nblk, Pm, st);
-                else if (ntile <= 12) e = vty_launch<12, 768>(N, w, nm, nblk, Pm, st);
-                else e = vty_launch<16, 512>(N, w, nm, nblk, Pm, st);
+                if (ntile <= 4) e = vty_launch<2, 768>(N, w, nm, nblk, Pm, st);
+                else if (ntile <= 8) e = vty_launch<4, 768>(N, w, nm, nblk, Pm, st);
+                else if (ntile <= 12) e = vty_launch<6, 768>(N, w, nm, nblk, Pm, st);
+                else e = vty_launch<8, 512>(N, w, nm, nblk, Pm, st);
                 if (e != cudaSuccess) return e;
             }
             ProjOut o{};
             for (int m = 0; m < n_mats; ++m) o.r[m] = out.r[m] + i0 + (int64_t)j0 * k;
             const int64_t tot = (int64_t)n_mats * ka * kb;
-            reduce_partials_kernel<<<(int)((tot + 255) / 256), 256, 0, st>>>(partial, nblk, n_mats, ka, kb, kap, kbp,
-                                                                               o, k);
+            reduce_partials_kernel<<<(int)((tot + 31) / 32), dim3(32, RED_SEG), 0, st>>>(partial, nblk, n_mats, ka, kb, kap,
+                                                                                       kbp, o, k);
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }
@@ -755,12 +959,14 @@ cudaError_t launch_gram_schmidt(double *V, int64_t N, int k, int64_t ldv, int pa
     double *part = work;
     double *Cm = part + (size_t)nblk * rows_max * GS_B;
     double *rinv = Cm + (size_t)rows_max * GS_B;
-    const size_t smem = sizeof(double) * (size_t)2 * (GS_WIN + GS_B) * GS_LDR;
-    cudaError_t e = cudaFuncSetAttribute(gs_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = sizeof(double) * (size_t)GS_STAGES * (GS_WIN + GS_B) * GS_LDR;
+    const bool pairs = (reinterpret_cast<uintptr_t>(V) & 15) == 0 && (ldv & 1) == 0;
+    auto gram = pairs ? gs_gram_kernel<true> : gs_gram_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int64_t n_chunks = (N + 31) / 32;
     const int64_t per = (n_chunks + nblk - 1) / nblk;
-    const int ugrid = (int)((N + 127) / 128);  // 128 rows per 256-thread CTA
+    const int ugrid = (int)((N + 16 * GS_UW - 1) / (16 * GS_UW));
     passes = std::max(passes, 1);
     for (int j0 = 0; j0 < k; j0 += GS_B) {
         const int b = std::min(GS_B, k - j0);
@@ -768,12 +974,12 @@ cudaError_t launch_gram_schmidt(double *V, int64_t N, int k, int64_t ldv, int pa
         for (int pass = 0; pass < passes; ++pass) {
             for (int x0 = 0; x0 < j0 + b; x0 += GS_WIN) {
                 const int w = std::min(GS_WIN, j0 + b - x0);
-                gs_gram_kernel<<<nblk, GS_THREADS, smem, st>>>(V, N, ldv, x0, w, j0, b, rows_c, per, part);
+                gram<<<nblk, GS_THREADS, smem, st>>>(V, N, ldv, x0, w, j0, b, rows_c, per, part);
             }
             const int64_t tot = (int64_t)rows_c * GS_B;
-            gs_reduce_kernel<<<(int)std::min<int64_t>((tot + 255) / 256, 1024), 256, 0, st>>>(part, nblk, rows_c, Cm);
-            gs_chol_kernel<<<1, 256, 0, st>>>(Cm, j0, b, rinv);
-            gs_update_kernel<<<ugrid, 256, 0, st>>>(V, N, ldv, j0, b, Cm, rinv);
+            gs_reduce_kernel<<<(int)((tot + 31) / 32), dim3(32, RED_SEG), 0, st>>>(part, nblk, rows_c, Cm);
+            gs_chol_kernel<<<1, GS_CT, 0, st>>>(Cm, j0, b, rinv);
+            gs_update_kernel<<<ugrid, 32 * GS_UW, 0, st>>>(V, N, ldv, j0, b, Cm, rinv);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
