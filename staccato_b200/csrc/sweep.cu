@@ -507,7 +507,11 @@ __device__ void factor_global(T *A, int64_t lda, int n, int ldp, unsigned char *
             PL.grp = 0;
         }
         __syncthreads();
-        panel_factor_par<T, RPT>(P, ldp, m, nbc, s_perm, s_pivlg, s_mdst, s_msrc, PL, j0, X);
+        if constexpr (std::is_same<T, float2>::value)  // the u region is free until the trailing update
+            panel_factor_32<RPT>(P, ldp, m, nbc, s_perm, reinterpret_cast<int *>(sm + L.pos), s_pivlg, s_mdst, s_msrc, PL, j0,
+                                  *reinterpret_cast<PanelXchg32 *>(sm + L.u));
+        else
+            panel_factor_par<T, RPT>(P, ldp, m, nbc, s_perm, s_pivlg, s_mdst, s_msrc, PL, j0, X);
         const int nmoved = PL.nmoved;
         for (int c = warp; c < nbc; c += NW)
             for (int i = lane; i < m; i += 32) A[(j0 + i) + (j0 + c) * lda] = P[s_perm[i] + (int64_t)c * ldp];

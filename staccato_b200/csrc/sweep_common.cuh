@@ -251,6 +251,164 @@ __device__ void panel_factor_par(T *P, int ldp, int m, int ncols, int *s_perm, i
     __syncthreads();
 }
 
+// ---- complex-FP32 panel ------------------------------------------------------------------------
+// The same factorisation as panel_factor_par, entry by entry, with a shorter chain between the columns: one
+// reduction on the value's bits (redux) instead of five rounds of three shuffles, one candidate a warp read by
+// lanes instead of eight by every thread, the reciprocal computed by every lane for its own candidate while the
+// reduction runs, and no divergent branch on the common path (ties and NaN have a path of their own).
+// (The rows in registers, as in sweep_lu64.cu, made the kernels 24 % slower: 128 registers a thread for two
+// rows of 32 columns, eight copies of the step for the shrinking width.)
+struct PanelXchg32 {
+    int4 cand[2][NW];     // key (bits of |re| + |im|, plus 1; 0: none), row, 1 if a NaN or a tie
+    float2 inv[2][NW];    // reciprocal of the candidate
+    int first;
+};
+
+__device__ __forceinline__ float2 recip_uniform(float2 z) {  // CT<float2>::recip, both cases in one sequence
+    const bool xb = fabsf(z.x) >= fabsf(z.y);
+    const float p = xb ? z.x : z.y, q = xb ? z.y : z.x;
+    const float t = q / p, d = p + q * t;
+    const float u = 1.0f / d, v = t / d;
+    return xb ? make_float2(u, -v) : make_float2(v, -u);
+}
+
+// s_lg: m ints of work space.  Outputs as panel_factor_par's.
+template <int RPT>
+__device__ __forceinline__ void panel_factor_32(float2 *P, int ldp, int m, int ncols, int *s_perm, int *s_lg,
+                                                int *s_pivlg, int *s_mdst, int *s_msrc, PanelLists &PL, int info_off,
+                                                PanelXchg32 &X) {
+    using C = CT<float2>;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned done = 0;
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+        const int ph = tid + k * NT;
+        if (ph >= m) done |= 1u << k;
+        else s_perm[ph] = s_lg[ph] = ph;
+    }
+    for (int jj = 0; jj < ncols; ++jj) {
+        const int buf = jj & 1;
+        unsigned kv[RPT], key = 0;
+        float2 cur[RPT], val = make_float2(1.0f, 0.5f);
+        bool odd = false;
+        int brr = 0;
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) {
+            const bool act = !((done >> k) & 1u);
+            cur[k] = act ? P[tid + k * NT + jj * ldp] : make_float2(0.f, 0.f);
+            const float v = C::abs1(cur[k]);
+            odd = odd || v != v;
+            kv[k] = act && v == v ? __float_as_uint(v) + 1u : 0u;
+            odd = odd || (k > 0 && kv[k] == key && key != 0);
+            if (kv[k] > key) {
+                key = kv[k];
+                brr = k;
+                val = cur[k];
+            }
+        }
+        const unsigned mk = __reduce_max_sync(FULL_MASK, key);
+        const float2 rec = recip_uniform(val);
+        const unsigned who = __ballot_sync(FULL_MASK, key != 0 && key == mk);
+        const int flag = __any_sync(FULL_MASK, odd) || (who & (who - 1));
+        if (lane == (who ? __ffs(who) - 1 : 0)) {
+            X.cand[buf][warp] = make_int4((int)key, 0, tid + brr * NT, flag);
+            X.inv[buf][warp] = rec;
+        }
+        __syncthreads();
+        const int4 c = lane < NW ? X.cand[buf][lane] : make_int4(0, 0, 0, 0);
+        unsigned bk = __reduce_max_sync(FULL_MASK, (unsigned)c.x);
+        const unsigned w = __ballot_sync(FULL_MASK, (unsigned)c.x == bk && c.x != 0);
+        const bool slow = __any_sync(FULL_MASK, c.w) || (w & (w - 1));
+        const int wl = w ? __ffs(w) - 1 : 0;
+        int bph = __shfl_sync(FULL_MASK, c.z, wl);
+        float2 iv = X.inv[buf][wl];
+        bool nz = true;
+        if (slow || bk <= 1) {
+            // IZAMAX takes the smallest logical row of the largest value and starts from the first entry: a NaN
+            // there is the pivot, all-NaN likewise; a zero pivot interchanges nothing
+            if (tid == 0) X.first = 0;
+            __syncthreads();
+            const int first = s_perm[jj];
+            int lg = INT_MAX, kb = 0;
+#pragma unroll
+            for (int k = 0; k < RPT; ++k) {
+                const int ph = tid + k * NT;
+                if (kv[k] != 0 && kv[k] == mk && s_lg[ph] < lg) {
+                    lg = s_lg[ph];
+                    kb = k;
+                }
+                if (ph == first) {
+                    const float v = C::abs1(cur[k]);
+                    if (v != v) X.first = 1;
+                }
+            }
+            const int mn = __reduce_min_sync(FULL_MASK, lg);
+            if (mn == INT_MAX ? lane == 0 : lg == mn) X.cand[buf][warp] = make_int4((int)mk, 0, tid + kb * NT, 0);
+            __syncthreads();
+            bk = 0;
+            bph = first;
+            for (int i = 0; i < NW; ++i) {
+                const int4 d = X.cand[buf][i];
+                if ((unsigned)d.x > bk || ((unsigned)d.x == bk && d.x != 0 && s_lg[d.z] < s_lg[bph])) {
+                    bk = (unsigned)d.x;
+                    bph = d.z;
+                }
+            }
+            if (X.first || bk <= 1) bph = first;
+            const float2 piv = P[bph + jj * ldp];
+            nz = piv.x != 0.0f || piv.y != 0.0f;
+            iv = nz ? C::recip(piv) : C::zero();
+            __syncthreads();  // s_lg, s_perm and the column are read; they change below
+        }
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) {
+            const int ph = tid + k * NT;
+            if (ph == bph) done |= 1u << k;
+            if ((done >> k) & 1u) continue;
+            float2 l = cur[k];
+            if (nz) {
+                l = C::mul(l, iv);
+                P[ph + jj * ldp] = l;
+            }
+            // rank-1 update of this row, four columns per batch so the shared-memory loads
+            // overlap (each entry still receives exactly this column's update)
+            int cc = jj + 1;
+            for (; cc + 4 <= ncols; cc += 4) {
+                float2 v[4], u[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    v[t] = P[ph + (cc + t) * ldp];
+                    u[t] = P[bph + (cc + t) * ldp];
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) P[ph + (cc + t) * ldp] = C::subm(v[t], l, u[t]);
+            }
+            for (; cc < ncols; ++cc) P[ph + cc * ldp] = C::subm(P[ph + cc * ldp], l, P[bph + cc * ldp]);
+        }
+        if (tid == NT - 1) {
+            // the interchange of logical rows jj and lg[bph]
+            const int first = s_perm[jj], lgp = s_lg[bph];
+            s_perm[lgp] = first;
+            s_lg[first] = lgp;
+            s_perm[jj] = bph;
+            s_lg[bph] = jj;
+            s_pivlg[jj] = lgp;
+            if (!nz && PL.info == 0) PL.info = info_off + jj + 1;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+        const int l = tid + k * NT;
+        if (l < m && s_perm[l] != l) {
+            const int e = atomicAdd(&PL.nmoved, 1);
+            s_mdst[e] = l;
+            s_msrc[e] = s_perm[l];
+        }
+    }
+    __syncthreads();
+}
+
 // r = b - A(w) x in FP64 with A(w) re-assembled from K, M, D (the FP64 assembly arithmetic),
 // written permuted and rounded to FP32 into B32 (B32[pos[i]] = r[i]) for the next correction.
 // Thread t owns rows t + k*NT; right-hand sides are processed four at a time; the column

@@ -87,7 +87,8 @@ constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >
 
 static_assert(TN % 16 == 0 && TN >= 16 && TN <= 256, "N of an M = 128 MMA");
 static_assert(TMEM_COLS >= 32 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "TMEM allocations are powers of two >= 32");
-static_assert(OP_BYTES >= (512 | 1) * NB * 8, "the panel of an n = 512 system fits the operand region");
+constexpr int PANEL_XCHG = ((int)sizeof(PanelXchg32) + 255) / 256 * 256;  // the panel factorisation's exchange
+static_assert(OP_BYTES >= (512 | 1) * NB * 8 + PANEL_XCHG, "the panel of an n = 512 system fits the operand region");
 
 // Byte offset of element (row, k) in one operand piece: K-major with the 128-byte swizzle.  A
 // row's 64 bf16 fill one 128-byte line, 8-row groups are 1024 bytes apart (SBO), and the 16-byte
@@ -919,7 +920,9 @@ __device__ __forceinline__ void factor_tc(float2 *A, int n, int lda, int ldp, un
         ++S.panels;
         __syncthreads();
         if (aborted(s_abort)) return;
-        panel_factor_par<float2, RPT>(P, ldp, m, nbc, s_perm, s_pivlg, s_mdst, s_msrc, PL, j0, X);
+        // the exchange lies in the operand region past the panel; the pos region is free until the refinement
+        panel_factor_32<RPT>(P, ldp, m, nbc, s_perm, reinterpret_cast<int *>(sm + L.pos), s_pivlg, s_mdst, s_msrc, PL, j0,
+                              *reinterpret_cast<PanelXchg32 *>(sm + L.op + OP_BYTES - PANEL_XCHG));
         const int nmoved = PL.nmoved;
         for (int c = warp; c < nbc; c += NW)
             for (int i = lane; i < m; i += 32) A[(j0 + i) + (int64_t)(j0 + c) * lda] = P[s_perm[i] + (int64_t)c * ldp];
