@@ -5,7 +5,8 @@
 // CTA's global scratch slot (or A in the caller's LU buffer), then per 16-column panel
 //   1. panel   thread t loads row t's 16 entries into registers and keeps them there for the 16
 //              elimination steps.  A step: two warp reductions (redux) find the pivot, every
-//              warp's candidate publishes its row in shared memory before the one CTA barrier, and
+//              warp's candidate publishes its row in shared memory before the one CTA barrier (from
+//              eight warps on the pivot's owner alone, behind a second one), and
 //              all rows take the rank-1 update from registers and the published row.  Rows are not
 //              moved: a logical permutation (s_perm) follows LAPACK's interchanges.  The multipliers
 //              go to the shared-memory panel P (physical row order), the U rows to the matrix.
@@ -27,12 +28,12 @@
 //
 // What bounds it: the chain of pivot steps (about 1300 cycles a column alone: reduction, reciprocal,
 // publishing the row, scaling) at orders up to about 200, with the FP64 pipe in the Schur updates above.
-// 128 registers a thread keep two (n <= 256), four (n <= 128) or five (n <= 64) systems an SM, so that
+// 128 registers a thread keep two (n <= 256), four (n <= 128) or six (n <= 64) systems an SM, so that
 // one system's pivot chain overlaps the others' Schur updates.
 // Measured on a B200, whole sweeps, against the kernels that it replaced (whole matrix in shared
 // memory, unblocked, up to n of about 112; 16-column panels with register-tiled fused multiply-adds,
-// one system an SM, above): n = 64, 500 systems, 318 -> 122 us; n = 189, 1000 systems, 4.9 -> 2.5 ms;
-// n = 256, r = 8, 2048 systems, 17.1 -> 9.6 ms.
+// one system an SM, above): n = 64, 500 systems, 318 -> 122 us; n = 189, 1000 systems, 4.9 -> 2.3 ms;
+// n = 256, r = 8, 2048 systems, 17.0 -> 9.3 ms.
 #include <algorithm>
 #include <climits>
 
@@ -140,12 +141,21 @@ struct Exchange {
 // 64-bit key a row (value bits + 1; 0 for none) with ties and NaNs in a path of their own, and the
 // reciprocal, the longest part, computed by every lane for its own entry before the barrier, where the
 // reduction and the previous step's update of the columns past the next one run in its shadow.
+// Warps without a row of the panel (tid >= m) only follow the pivots: with several systems an SM the steps are
+// bound by instruction issue, and most panels are shorter than the thread count: 1000 systems of order 189 went
+// from 2.30 to 2.21 ms with it, of order 150 from 1.49 to 1.40 ms.
 template <int NT_, int W>
 __device__ __forceinline__ void panel_steps(double2 (&a)[NB], int jj0, int jj1, int nbc, int j0, double2 *A,
                                             int64_t lda, double2 *P, int ldp, const Exchange<NT_> &X, int *s_pivlg,
-                                            int *s_perm, Shared &S, bool &done) {
+                                            int *s_perm, Shared &S, int m, bool &done) {
     constexpr int NWT = NT_ / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // LATE: the pivot's row is published by its owner, behind a second barrier, instead of every warp's
+    // candidate's before the first.  A lane's 16-byte stores take the shared-memory datapath as long as a whole
+    // warp's (16 cycles each): with eight warps or more they cost more than the barrier (order 189: 2.21 -> 2.18 ms,
+    // 256 with r = 8: 2.67 -> 2.63 ms a 592 systems).
+    constexpr bool LATE = NWT >= 8;
+    const bool live = warp * 32 < m;
     double2 lp = make_double2(0.0, 0.0);
     const double2 *up = nullptr;  // the previous step's pivot row
     for (int jj = jj0; jj < jj1; ++jj) {
@@ -157,23 +167,32 @@ __device__ __forceinline__ void panel_steps(double2 (&a)[NB], int jj0, int jj1, 
 #pragma unroll
             for (int c = 0; c < W; ++c) rw[w * NB + c] = a[c];
         };
-        const double v = cabs1(a[0]);
-        const bool nan = !done && v != v;
-        const unsigned long long key = done || v != v ? 0 : (unsigned long long)__double_as_longlong(v) + 1;
-        const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-        const unsigned bh = __reduce_max_sync(FULL_MASK, hi);
-        const double2 rec = crecip_uniform(key ? a[0] : make_double2(1.0, 0.5));  // off the zero operands' path
-        if (jj > jj0) {
+        bool nan = false;
+        unsigned long long key = 0;
+        unsigned hi = 0, lo = 0, bh = 0;
+        double2 rec = make_double2(0.0, 0.0);
+        if (live) {
+            const double v = cabs1(a[0]);
+            nan = !done && v != v;
+            key = done || v != v ? 0 : (unsigned long long)__double_as_longlong(v) + 1;
+            hi = (unsigned)(key >> 32);
+            lo = (unsigned)key;
+            bh = __reduce_max_sync(FULL_MASK, hi);
+            rec = crecip_uniform(key ? a[0] : make_double2(1.0, 0.5));  // off the zero operands' path
+            if (jj > jj0) {
 #pragma unroll
-            for (int c = 1; c + 1 < W; ++c) a[c] = csubmul(a[c + 1], lp, up[c + 1]);
-        }
-        const unsigned who = __ballot_sync(FULL_MASK, key != 0 && hi == bh);
-        // flag: a NaN, or rows of equal value (high words compared), for the path below to sort out
-        const int odd = __any_sync(FULL_MASK, nan) || (who & (who - 1));
-        if (lane == (who ? __ffs(who) - 1 : 0)) {
-            cand[warp] = make_int4((int)lo, (int)hi, tid, odd);
-            inv[warp] = rec;
-            store_row(warp);
+                for (int c = 1; c + 1 < W; ++c) a[c] = csubmul(a[c + 1], lp, up[c + 1]);
+            }
+            const unsigned who = __ballot_sync(FULL_MASK, key != 0 && hi == bh);
+            // flag: a NaN, or rows of equal value (high words compared), for the path below to sort out
+            const int odd = __any_sync(FULL_MASK, nan) || (who & (who - 1));
+            if (lane == (who ? __ffs(who) - 1 : 0)) {
+                cand[warp] = make_int4((int)lo, (int)hi, tid, odd);
+                if constexpr (!LATE) {
+                    inv[warp] = rec;
+                    store_row(warp);
+                }
+            }
         }
         __syncthreads();
         unsigned long long bkey;
@@ -214,8 +233,8 @@ __device__ __forceinline__ void panel_steps(double2 (&a)[NB], int jj0, int jj1, 
             if (tid == first && nan) S.first = 1;
             const unsigned bl = __reduce_max_sync(FULL_MASK, hi == bh ? lo : 0u);
             const int lg = key != 0 && hi == bh && lo == bl ? X.lg[tid] : INT_MAX;
-            const int m = __reduce_min_sync(FULL_MASK, lg);
-            if (m == INT_MAX ? lane == 0 : lg == m) {
+            const int low = __reduce_min_sync(FULL_MASK, lg);
+            if (low == INT_MAX ? lane == 0 : lg == low) {
                 cand[warp] = make_int4((int)lo, (int)hi, tid, 0);
                 inv[warp] = rec;
                 store_row(warp);
@@ -243,14 +262,23 @@ __device__ __forceinline__ void panel_steps(double2 (&a)[NB], int jj0, int jj1, 
             }
             __syncthreads();
             nz = rw[wl * NB].x != 0.0 || rw[wl * NB].y != 0.0;
+        } else if constexpr (LATE) {
+            wl = 0;
+            if (tid == bph) {
+                inv[0] = rec;
+                store_row(0);
+            }
+            __syncthreads();
         }
         const double2 *pr = rw + wl * NB;
-        lp = nz ? cmul(a[0], inv[wl]) : a[0];
-        a[0] = csubmul(a[1], lp, pr[1]);
-        done = done || tid == bph;
-        if (!done) P[tid + jj * ldp] = lp;
-        up = pr;
-        if (warp == (wl + 1) % NWT) {
+        if (live) {
+            lp = nz ? cmul(a[0], inv[wl]) : a[0];
+            a[0] = csubmul(a[1], lp, pr[1]);
+            done = done || tid == bph;
+            if (!done) P[tid + jj * ldp] = lp;
+            up = pr;
+        }
+        if (warp == (m < NT_ - 31 ? NWT - 1 : (wl + 1) % NWT)) {  // a warp without rows, if there is one
             if (lane < nbc - jj) A[(j0 + jj) + (int64_t)(j0 + jj + lane) * lda] = pr[lane];
             if (lane == 0) {
                 // the interchange of logical rows jj and lg[bph]
@@ -263,7 +291,7 @@ __device__ __forceinline__ void panel_steps(double2 (&a)[NB], int jj0, int jj1, 
             }
         }
     }
-    if (jj1 > jj0) {
+    if (live && jj1 > jj0) {
 #pragma unroll
         for (int c = 1; c + 1 < W; ++c) a[c] = csubmul(a[c + 1], lp, up[c + 1]);
     }
@@ -304,10 +332,11 @@ __device__ __forceinline__ void factor(double2 *A, int64_t lda, double2 *B, int6
                 X.at[tid] = tid;
                 X.lg[tid] = tid;
             }
-            panel_steps<NT_, 16>(a, 0, min(4, nbc), nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, done);
-            panel_steps<NT_, 12>(a, 4, min(8, nbc), nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, done);
-            panel_steps<NT_, 8>(a, 8, min(12, nbc), nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, done);
-            panel_steps<NT_, 4>(a, 12, nbc, nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, done);
+            if (warp * 32 >= m && lane == 0) X.cand[warp] = X.cand[NWT + warp] = make_int4(0, 0, tid, 0);
+            panel_steps<NT_, 16>(a, 0, min(4, nbc), nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, m, done);
+            panel_steps<NT_, 12>(a, 4, min(8, nbc), nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, m, done);
+            panel_steps<NT_, 8>(a, 8, min(12, nbc), nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, m, done);
+            panel_steps<NT_, 4>(a, 12, nbc, nbc, j0, A, lda, P, ldp, X, s_pivlg, s_perm, S, m, done);
         }
         __syncthreads();
         if (tid < m) {
