@@ -438,10 +438,10 @@ int mixed_class(const srom_handle *h, int n, int r, int flags) {
     return 2 * (srom::fp64_smem_bytes(n, r) + 1024) <= (size_t)h->max_smem_optin + 1024 ? 0 : 1;
 }
 
-// SROM_MIXED_AUTO: the tensor-core kernel from this order up (without a measurement).  On the
-// batching shapes it is 2-8 % faster than the CUDA-core kernel from n = 384 on and 8 % slower at
-// n = 256 (r = 8); the factorisation's panel, inverse blocks and per-column work weigh more at
-// smaller orders.
+// SROM_MIXED_AUTO: the tensor-core kernel from this order up (without a measurement).  592
+// systems, CUDA-core against tensor-core kernel: n = 512, r = 4, 20.4 / 14.4 ms; 384, r = 4, 9.8 / 8.4;
+// 320, r = 1, 6.5 / 5.5; 256, r = 4, 3.63 / 3.62; 160, r = 4, 1.58 / 1.81.  Between 200 and 320 it
+// depends on r, and srom_tune measures it.
 constexpr int TC_AUTO_MIN_N = 320;
 
 // Whether a mixed system of the global class runs on the tensor-core kernel.

@@ -473,11 +473,25 @@ struct GlobalSmem {
         moved = ipiv + up((size_t)ldp * 4);
         dinv = moved + up((size_t)2 * 2 * NB32 * 4);
         u = dinv + (big ? 0 : up((size_t)ldp * 16));      // reciprocals of diag(U), mixed form
+        static_assert(sizeof(PanelXchg32) <= (size_t)NW * 2048, "the panel's exchange fits the u region");
         panel = u + up((size_t)NW * 2048);                // per warp NB x CWG complex
         total = panel + (big ? up((size_t)32 * 33 * 16)   // the solve's diagonal tile
                              : up((size_t)ldp * 256));    // ldp x 16 double2 == ldp x 32 float2
     }
 };
+
+// panel_factor_32 as a function of its own, its arguments shared-memory offsets so that its accesses are known to
+// be shared ones: inlined into this kernel the same code took 1.3 times as long a column (256 rows: 1870 cycles
+// against 1400; in the tensor-core kernel the inlined form is the faster one).
+extern __shared__ __align__(256) unsigned char panel_sm[];
+template <int RPT>
+__device__ __noinline__ void panel_call(unsigned p_off, int ldp, int m, int ncols, unsigned perm_off, unsigned lg_off,
+                                        int *s_pivlg, unsigned moved_off, PanelLists &PL, int info_off, unsigned x_off) {
+    int *moved = reinterpret_cast<int *>(panel_sm + moved_off);
+    panel_factor_32<RPT>(reinterpret_cast<float2 *>(panel_sm + p_off), ldp, m, ncols,
+                         reinterpret_cast<int *>(panel_sm + perm_off), reinterpret_cast<int *>(panel_sm + lg_off), s_pivlg,
+                         moved, moved + 2 * NB32, PL, info_off, *reinterpret_cast<PanelXchg32 *>(panel_sm + x_off));
+}
 
 // Blocked LU of the system already assembled in A (n x n, lda).  B (smem, ld n, nrhs
 // columns, may be null) receives the interchanges; s_ptot (smem) the composite row
@@ -508,8 +522,8 @@ __device__ void factor_global(T *A, int64_t lda, int n, int ldp, unsigned char *
         }
         __syncthreads();
         if constexpr (std::is_same<T, float2>::value)  // the u region is free until the trailing update
-            panel_factor_32<RPT>(P, ldp, m, nbc, s_perm, reinterpret_cast<int *>(sm + L.pos), s_pivlg, s_mdst, s_msrc, PL, j0,
-                                  *reinterpret_cast<PanelXchg32 *>(sm + L.u));
+            panel_call<RPT>((unsigned)L.panel, ldp, m, nbc, (unsigned)L.perm, (unsigned)L.pos, s_pivlg, (unsigned)L.moved,
+                            PL, j0, (unsigned)L.u);
         else
             panel_factor_par<T, RPT>(P, ldp, m, nbc, s_perm, s_pivlg, s_mdst, s_msrc, PL, j0, X);
         const int nmoved = PL.nmoved;

@@ -252,15 +252,25 @@ __device__ void panel_factor_par(T *P, int ldp, int m, int ncols, int *s_perm, i
 }
 
 // ---- complex-FP32 panel ------------------------------------------------------------------------
-// The same factorisation as panel_factor_par, entry by entry, with a shorter chain between the columns: one
-// reduction on the value's bits (redux) instead of five rounds of three shuffles, one candidate a warp read by
-// lanes instead of eight by every thread, the reciprocal computed by every lane for its own candidate while the
-// reduction runs, and no divergent branch on the common path (ties and NaN have a path of their own).
-// (The rows in registers, as in sweep_lu64.cu, made the kernels 24 % slower: 128 registers a thread for two
-// rows of 32 columns, eight copies of the step for the shrinking width.)
+// The same factorisation as panel_factor_par, entry by entry, eight columns at a time.  A thread holds its rows'
+// eight entries in registers for the group's steps (shifted by one column a step, so that the code of a step is
+// there once); the panel's further columns take the group's eight updates together, in the same order, in one
+// pass: with an update of the whole row from shared memory in every step, that traffic was most of the panel's
+// time (n = 512: 16 bytes an entry and step; 2130 cycles a column, now 1760, at n = 320 1860 and 1660 in the
+// tensor-core kernel; 592 systems, whole sweep: n = 320 5.80 -> 5.52 ms, n = 512, r = 4, 15.1 -> 14.4 ms, CUDA-core
+// n = 200 2.52 -> 2.41 ms, n = 256, r = 4, 3.77 -> 3.63 ms).
+// The chain between the columns: one reduction on the value's bits (redux), one candidate a warp with its
+// row and its reciprocal, computed by every lane for its own candidate while the reduction runs, published before
+// the step's one barrier, and no divergent branch on the common path (ties and NaN have a path of their own).
+// Warps without rows only follow.
+// (All 32 columns of the rows in registers made the kernels 24 % slower: 128 registers a thread for two rows,
+// eight copies of the step for the shrinking width.)
+constexpr int PG = 8;  // columns of a group
 struct PanelXchg32 {
-    int4 cand[2][NW];     // key (bits of |re| + |im|, plus 1; 0: none), row, 1 if a NaN or a tie
-    float2 inv[2][NW];    // reciprocal of the candidate
+    float2 row[2][NW][PG];          // the candidates' rows, two buffers by the step's parity
+    float2 u[NB32 - PG][PG];        // the group's U entries of the further columns
+    int4 cand[2][NW];               // key (bits of |re| + |im|, plus 1; 0: none), row, 1 if a NaN or a tie
+    float2 inv[2][NW];              // reciprocal of the candidate
     int first;
 };
 
@@ -272,13 +282,14 @@ __device__ __forceinline__ float2 recip_uniform(float2 z) {  // CT<float2>::reci
     return xb ? make_float2(u, -v) : make_float2(v, -u);
 }
 
-// s_lg: m ints of work space.  Outputs as panel_factor_par's.
+// s_lg: m ints of work space; X 16-byte aligned.  Outputs as panel_factor_par's.
 template <int RPT>
 __device__ __forceinline__ void panel_factor_32(float2 *P, int ldp, int m, int ncols, int *s_perm, int *s_lg,
                                                 int *s_pivlg, int *s_mdst, int *s_msrc, PanelLists &PL, int info_off,
                                                 PanelXchg32 &X) {
     using C = CT<float2>;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool live = warp * 32 < m;
     unsigned done = 0;
 #pragma unroll
     for (int k = 0; k < RPT; ++k) {
@@ -286,114 +297,195 @@ __device__ __forceinline__ void panel_factor_32(float2 *P, int ldp, int m, int n
         if (ph >= m) done |= 1u << k;
         else s_perm[ph] = s_lg[ph] = ph;
     }
-    for (int jj = 0; jj < ncols; ++jj) {
-        const int buf = jj & 1;
-        unsigned kv[RPT], key = 0;
-        float2 cur[RPT], val = make_float2(1.0f, 0.5f);
-        bool odd = false;
-        int brr = 0;
+    if (!live && lane == 0) X.cand[0][warp] = X.cand[1][warp] = make_int4(0, 0, tid, 0);
+    for (int g0 = 0; g0 < ncols; g0 += PG) {
+        const int gw = min(PG, ncols - g0);
+        float2 a[RPT][PG];
 #pragma unroll
-        for (int k = 0; k < RPT; ++k) {
-            const bool act = !((done >> k) & 1u);
-            cur[k] = act ? P[tid + k * NT + jj * ldp] : make_float2(0.f, 0.f);
-            const float v = C::abs1(cur[k]);
-            odd = odd || v != v;
-            kv[k] = act && v == v ? __float_as_uint(v) + 1u : 0u;
-            odd = odd || (k > 0 && kv[k] == key && key != 0);
-            if (kv[k] > key) {
-                key = kv[k];
-                brr = k;
-                val = cur[k];
+        for (int k = 0; k < RPT; ++k)
+#pragma unroll
+            for (int c = 0; c < PG; ++c)
+                a[k][c] = !((done >> k) & 1u) && c < gw ? P[tid + k * NT + (g0 + c) * ldp] : make_float2(0.f, 0.f);
+        for (int jj = g0; jj < g0 + gw; ++jj) {
+            const int buf = jj & 1;
+            unsigned kv[RPT], key = 0, mk = 0;
+            float2 rec = make_float2(0.f, 0.f);
+            int brr = 0;
+            auto store_row = [&](int w, int kr) {
+#pragma unroll
+                for (int c = 0; c < PG; c += 2) {
+                    float2 v = a[0][c], v1 = a[0][c + 1];
+#pragma unroll
+                    for (int k = 1; k < RPT; ++k) {
+                        v = kr == k ? a[k][c] : v;
+                        v1 = kr == k ? a[k][c + 1] : v1;
+                    }
+                    *reinterpret_cast<float4 *>(&X.row[buf][w][c]) = make_float4(v.x, v.y, v1.x, v1.y);
+                }
+            };
+#pragma unroll
+            for (int k = 0; k < RPT; ++k) kv[k] = 0;
+            if (live) {
+                float2 val = make_float2(1.0f, 0.5f);
+                bool odd = false;
+#pragma unroll
+                for (int k = 0; k < RPT; ++k) {
+                    const bool act = !((done >> k) & 1u);
+                    const float v = C::abs1(a[k][0]);
+                    odd = odd || (act && v != v);
+                    kv[k] = act && v == v ? __float_as_uint(v) + 1u : 0u;
+                    odd = odd || (k > 0 && kv[k] == key && key != 0);
+                    if (kv[k] > key) {
+                        key = kv[k];
+                        brr = k;
+                        val = a[k][0];
+                    }
+                }
+                mk = __reduce_max_sync(FULL_MASK, key);
+                rec = recip_uniform(val);
+                const unsigned who = __ballot_sync(FULL_MASK, key != 0 && key == mk);
+                const int flag = __any_sync(FULL_MASK, odd) || (who & (who - 1));
+                if (lane == (who ? __ffs(who) - 1 : 0)) {
+                    X.cand[buf][warp] = make_int4((int)key, 0, tid + brr * NT, flag);
+                    X.inv[buf][warp] = rec;
+                    store_row(warp, brr);
+                }
             }
-        }
-        const unsigned mk = __reduce_max_sync(FULL_MASK, key);
-        const float2 rec = recip_uniform(val);
-        const unsigned who = __ballot_sync(FULL_MASK, key != 0 && key == mk);
-        const int flag = __any_sync(FULL_MASK, odd) || (who & (who - 1));
-        if (lane == (who ? __ffs(who) - 1 : 0)) {
-            X.cand[buf][warp] = make_int4((int)key, 0, tid + brr * NT, flag);
-            X.inv[buf][warp] = rec;
+            __syncthreads();
+            const int4 c4 = lane < NW ? X.cand[buf][lane] : make_int4(0, 0, 0, 0);
+            unsigned bk = __reduce_max_sync(FULL_MASK, (unsigned)c4.x);
+            const unsigned w = __ballot_sync(FULL_MASK, (unsigned)c4.x == bk && c4.x != 0);
+            const bool slow = __any_sync(FULL_MASK, c4.w) || (w & (w - 1));
+            int wl = w ? __ffs(w) - 1 : 0;
+            int bph = __shfl_sync(FULL_MASK, c4.z, wl);
+            float2 iv = X.inv[buf][wl];
+            bool nz = true;
+            if (slow || bk <= 1) {
+                // IZAMAX takes the smallest logical row of the largest value and starts from the first entry: a NaN
+                // there is the pivot, all-NaN likewise; a zero pivot interchanges nothing
+                if (tid == 0) X.first = 0;
+                __syncthreads();
+                const int first = s_perm[jj];
+                int lg = INT_MAX, kb = 0;
+#pragma unroll
+                for (int k = 0; k < RPT; ++k) {
+                    const int ph = tid + k * NT;
+                    if (kv[k] != 0 && kv[k] == mk && s_lg[ph] < lg) {
+                        lg = s_lg[ph];
+                        kb = k;
+                    }
+                    if (ph == first) {
+                        const float v = C::abs1(a[k][0]);
+                        if (v != v) X.first = 1;
+                    }
+                }
+                const int mn = __reduce_min_sync(FULL_MASK, lg);
+                if (mn == INT_MAX ? lane == 0 : lg == mn) X.cand[buf][warp] = make_int4((int)mk, 0, tid + kb * NT, 0);
+                __syncthreads();
+                bk = 0;
+                bph = first;
+                for (int i = 0; i < NW; ++i) {
+                    const int4 d = X.cand[buf][i];
+                    if ((unsigned)d.x > bk || ((unsigned)d.x == bk && d.x != 0 && s_lg[d.z] < s_lg[bph])) {
+                        bk = (unsigned)d.x;
+                        bph = d.z;
+                    }
+                }
+                if (X.first || bk <= 1) bph = first;
+                wl = 0;
+                if (tid == bph % NT) store_row(0, bph / NT);
+                __syncthreads();  // s_lg and s_perm are read; they change below
+                const float2 piv = X.row[buf][0][0];
+                nz = piv.x != 0.0f || piv.y != 0.0f;
+                iv = nz ? C::recip(piv) : C::zero();
+            }
+            const float2 *pr = X.row[buf][wl];
+            if (live) {
+                float2 u[PG];
+#pragma unroll
+                for (int c = 0; c < PG; c += 2) {
+                    const float4 v = *reinterpret_cast<const float4 *>(pr + c);
+                    u[c] = make_float2(v.x, v.y);
+                    u[c + 1] = make_float2(v.z, v.w);
+                }
+#pragma unroll
+                for (int k = 0; k < RPT; ++k) {
+                    const int ph = tid + k * NT;
+                    if (ph == bph) done |= 1u << k;
+                    const float2 l = nz ? C::mul(a[k][0], iv) : a[k][0];
+                    if (!((done >> k) & 1u)) P[ph + jj * ldp] = l;
+#pragma unroll
+                    for (int c = 0; c + 1 < PG; ++c) a[k][c] = C::subm(a[k][c + 1], l, u[c + 1]);
+                }
+            }
+            if (warp == (m <= NT - 32 ? NW - 1 : (wl + 1) % NW)) {  // a warp without rows, if there is one
+                if (lane < g0 + gw - jj) P[bph + (jj + lane) * ldp] = pr[lane];
+                if (lane == 0) {
+                    // the interchange of logical rows jj and lg[bph]
+                    const int first = s_perm[jj], lgp = s_lg[bph];
+                    s_perm[lgp] = first;
+                    s_lg[first] = lgp;
+                    s_perm[jj] = bph;
+                    s_lg[bph] = jj;
+                    s_pivlg[jj] = lgp;
+                    if (!nz && PL.info == 0) PL.info = info_off + jj + 1;
+                }
+            }
         }
         __syncthreads();
-        const int4 c = lane < NW ? X.cand[buf][lane] : make_int4(0, 0, 0, 0);
-        unsigned bk = __reduce_max_sync(FULL_MASK, (unsigned)c.x);
-        const unsigned w = __ballot_sync(FULL_MASK, (unsigned)c.x == bk && c.x != 0);
-        const bool slow = __any_sync(FULL_MASK, c.w) || (w & (w - 1));
-        const int wl = w ? __ffs(w) - 1 : 0;
-        int bph = __shfl_sync(FULL_MASK, c.z, wl);
-        float2 iv = X.inv[buf][wl];
-        bool nz = true;
-        if (slow || bk <= 1) {
-            // IZAMAX takes the smallest logical row of the largest value and starts from the first entry: a NaN
-            // there is the pivot, all-NaN likewise; a zero pivot interchanges nothing
-            if (tid == 0) X.first = 0;
+        const int c0 = g0 + PG, nr = ncols - c0;
+        if (nr > 0) {
+            // the group's pivot rows in the further columns: a lane a column, the unit triangle
+            if (warp == 0 && lane < nr) {
+                int pv[PG];
+                float2 u[PG];
+#pragma unroll
+                for (int t = 0; t < PG; ++t) {
+                    pv[t] = s_perm[g0 + t];
+                    u[t] = P[pv[t] + (c0 + lane) * ldp];
+                }
+#pragma unroll
+                for (int q = 0; q + 1 < PG; ++q)
+#pragma unroll
+                    for (int t = q + 1; t < PG; ++t) u[t] = C::subm(u[t], P[pv[t] + (g0 + q) * ldp], u[q]);
+#pragma unroll
+                for (int t = 0; t < PG; ++t) {
+                    if (t > 0) P[pv[t] + (c0 + lane) * ldp] = u[t];
+                    X.u[lane][t] = u[t];
+                }
+            }
             __syncthreads();
-            const int first = s_perm[jj];
-            int lg = INT_MAX, kb = 0;
+            // the rows below, a thread a row, the group's columns in order
+            bool any = false;
+            float2 l[RPT][PG];
 #pragma unroll
             for (int k = 0; k < RPT; ++k) {
-                const int ph = tid + k * NT;
-                if (kv[k] != 0 && kv[k] == mk && s_lg[ph] < lg) {
-                    lg = s_lg[ph];
-                    kb = k;
-                }
-                if (ph == first) {
-                    const float v = C::abs1(cur[k]);
-                    if (v != v) X.first = 1;
-                }
-            }
-            const int mn = __reduce_min_sync(FULL_MASK, lg);
-            if (mn == INT_MAX ? lane == 0 : lg == mn) X.cand[buf][warp] = make_int4((int)mk, 0, tid + kb * NT, 0);
-            __syncthreads();
-            bk = 0;
-            bph = first;
-            for (int i = 0; i < NW; ++i) {
-                const int4 d = X.cand[buf][i];
-                if ((unsigned)d.x > bk || ((unsigned)d.x == bk && d.x != 0 && s_lg[d.z] < s_lg[bph])) {
-                    bk = (unsigned)d.x;
-                    bph = d.z;
-                }
-            }
-            if (X.first || bk <= 1) bph = first;
-            const float2 piv = P[bph + jj * ldp];
-            nz = piv.x != 0.0f || piv.y != 0.0f;
-            iv = nz ? C::recip(piv) : C::zero();
-            __syncthreads();  // s_lg, s_perm and the column are read; they change below
-        }
+                const bool act = !((done >> k) & 1u);
+                any = any || act;
 #pragma unroll
-        for (int k = 0; k < RPT; ++k) {
-            const int ph = tid + k * NT;
-            if (ph == bph) done |= 1u << k;
-            if ((done >> k) & 1u) continue;
-            float2 l = cur[k];
-            if (nz) {
-                l = C::mul(l, iv);
-                P[ph + jj * ldp] = l;
+                for (int t = 0; t < PG; ++t) l[k][t] = act ? P[tid + k * NT + (g0 + t) * ldp] : make_float2(0.f, 0.f);
             }
-            // rank-1 update of this row, four columns per batch so the shared-memory loads
-            // overlap (each entry still receives exactly this column's update)
-            int cc = jj + 1;
-            for (; cc + 4 <= ncols; cc += 4) {
-                float2 v[4], u[4];
+            if (any) {
+#pragma unroll 2
+                for (int c = 0; c < nr; ++c) {
+                    float2 v[RPT];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    v[t] = P[ph + (cc + t) * ldp];
-                    u[t] = P[bph + (cc + t) * ldp];
+                    for (int k = 0; k < RPT; ++k)
+                        if (!((done >> k) & 1u)) v[k] = P[tid + k * NT + (c0 + c) * ldp];
+#pragma unroll
+                    for (int t = 0; t < PG; t += 2) {
+                        const float4 u = *reinterpret_cast<const float4 *>(&X.u[c][t]);
+#pragma unroll
+                        for (int k = 0; k < RPT; ++k) {
+                            v[k] = C::subm(v[k], l[k][t], make_float2(u.x, u.y));
+                            v[k] = C::subm(v[k], l[k][t + 1], make_float2(u.z, u.w));
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < RPT; ++k)
+                        if (!((done >> k) & 1u)) P[tid + k * NT + (c0 + c) * ldp] = v[k];
                 }
-#pragma unroll
-                for (int t = 0; t < 4; ++t) P[ph + (cc + t) * ldp] = C::subm(v[t], l, u[t]);
             }
-            for (; cc < ncols; ++cc) P[ph + cc * ldp] = C::subm(P[ph + cc * ldp], l, P[bph + cc * ldp]);
-        }
-        if (tid == NT - 1) {
-            // the interchange of logical rows jj and lg[bph]
-            const int first = s_perm[jj], lgp = s_lg[bph];
-            s_perm[lgp] = first;
-            s_lg[first] = lgp;
-            s_perm[jj] = bph;
-            s_lg[bph] = jj;
-            s_pivlg[jj] = lgp;
-            if (!nz && PL.info == 0) PL.info = info_off + jj + 1;
         }
     }
     __syncthreads();

@@ -25,7 +25,7 @@
 // Intelligence Datatype For Higher-Precision Computations", 2019.)
 //
 // Data flow of one panel step j0 (matrix in the CTA's global scratch slot, L2-resident):
-//   A  panel: columns j0..j0+31 staged in shared memory and factored (panel_factor_par); the
+//   A  panel: columns j0..j0+31 staged in shared memory and factored (panel_factor_32); the
 //      factored panel is written back in logical row order; L11^-1 (unit lower, 32 x 32) is
 //      formed in shared memory; L21 is written to the CTA's A-operand buffer in global memory
 //      as ready-made tcgen05 operand tiles (three bf16 pieces, K-major core-matrix layout);
@@ -318,7 +318,9 @@ __device__ __noinline__ void assemble_fp32(float2 *A, int lda, const RomDev &R, 
 // forms columns j = w, w + 8, w + 16, w + 24 of both inverses together (lane i holds row i):
 // L11^-1 e_j by forward elimination (y_i -= L[i][k] y_k for k = j..bs-2, i > k) and U11^-1 e_j
 // by back substitution (y_k = (e_j - sum_{m>k} U[k][m] y_m) / U[k][k], k = j..0), the entry of
-// L or U and the pivot's reciprocal of each step shared by the four columns.  L11^-1 goes to
+// L or U and the pivot's reciprocal of each step shared by the four columns (the reciprocals formed
+// once, a lane its own diagonal entry, and the entries loaded a step ahead: 418 -> 272 thousand
+// cycles a system of n = 512).  L11^-1 goes to
 // shared memory (phase B) and both to the CTA's global inverse buffer (the correction solves),
 // 32 x 32 column-major with zeros outside bs x bs.
 __device__ __forceinline__ void build_inverses(const float2 *P, int ldp, const int *s_perm, int bs, float2 *s_linv,
@@ -331,8 +333,10 @@ __device__ __forceinline__ void build_inverses(const float2 *P, int ldp, const i
     float2 y[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) y[q] = (act && lane == warp + NW * q) ? make_float2(1.f, 0.f) : C::zero();
+    float2 nx = act && warp < bs ? P[pr + (int64_t)warp * ldp] : C::zero();  // one step ahead
     for (int k = warp; k < bs - 1; ++k) {
-        const float2 l = (act && lane > k) ? P[pr + (int64_t)k * ldp] : C::zero();
+        const float2 l = nx;
+        nx = act ? P[pr + (int64_t)(k + 1) * ldp] : C::zero();
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             const float2 yk = C::shfl(y[q], k, 32);
@@ -352,9 +356,14 @@ __device__ __forceinline__ void build_inverses(const float2 *P, int ldp, const i
         y[q] = C::zero();
         acc[q] = (act && lane == warp + NW * q) ? make_float2(1.f, 0.f) : C::zero();
     }
-    for (int k = min(warp + NW * (Q - 1), bs - 1); k >= 0; --k) {
-        const float2 u = act ? P[pr + (int64_t)k * ldp] : C::zero();  // U[lane][k]
-        const float2 rk = C::shfl(lane == k ? C::recip(u) : C::zero(), k, 32);
+    // the divisions once for all steps, a lane its own diagonal entry
+    const float2 rd = act ? C::recip(P[pr + (int64_t)lane * ldp]) : C::zero();
+    const int k0 = min(warp + NW * (Q - 1), bs - 1);
+    nx = act ? P[pr + (int64_t)k0 * ldp] : C::zero();
+    for (int k = k0; k >= 0; --k) {
+        const float2 u = nx;  // U[lane][k]
+        nx = act && k > 0 ? P[pr + (int64_t)(k - 1) * ldp] : C::zero();
+        const float2 rk = C::shfl(rd, k, 32);
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             if (k > warp + NW * q) continue;  // column j = warp + NW q starts at k = j
@@ -884,7 +893,7 @@ struct TcSolve {
 template <int RPT>
 __device__ __forceinline__ void factor_tc(float2 *A, int n, int lda, int ldp, unsigned char *sm, const TcSmem &L,
                                        unsigned char *abuf, unsigned char *bbuf, float2 *ginv, int *moves, PanelLists &PL,
-                                       PivotXchg<float> &X, int *s_pivlg, uint32_t tmem, const Bars &B, TcState &S,
+                                       int *s_pivlg, uint32_t tmem, const Bars &B, TcState &S,
                                        int *s_abort, int *err_flag) {
     float2 *P = reinterpret_cast<float2 *>(sm + L.op);
     int *s_perm = reinterpret_cast<int *>(sm + L.perm);
@@ -976,7 +985,6 @@ __global__ void __launch_bounds__(NT, 1) sweep_tc_kernel(GlobalArgs a) {
     __shared__ int s_item;
     __shared__ int s_pivlg[NB];
     __shared__ PanelLists PL;
-    __shared__ PivotXchg<float> Xx;
     __shared__ double s_dx[RMAX_MIXED];
     __shared__ int s_abort, s_phase;
     unsigned char *sm = sm_raw + ((1024u - (su32(sm_raw) & 1023u)) & 1023u);
@@ -1030,7 +1038,7 @@ __global__ void __launch_bounds__(NT, 1) sweep_tc_kernel(GlobalArgs a) {
         const int lda = tc_lda(n);
         assemble_fp32(A32, lda, R, w, wi.f);
         __syncthreads();
-        factor_tc<RPT>(A32, n, lda, a.ldp, sm, L, abuf, bbuf, ginv, moves, PL, Xx, s_pivlg, tmem, B, S, &s_abort,
+        factor_tc<RPT>(A32, n, lda, a.ldp, sm, L, abuf, bbuf, ginv, moves, PL, s_pivlg, tmem, B, S, &s_abort,
                        a.err_flag);
         __syncthreads();
         if (aborted(&s_abort)) {
