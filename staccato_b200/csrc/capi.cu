@@ -548,6 +548,10 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
         *rm = std::max(*rm, d.r);
         P.n_items[c] += d.F;
         P.flops[c] += lu_flops(d.n, d.r) * d.F;
+        // a row-kernel slot is laid out by its system's own sizes: the largest one, not the largest
+        // order with the largest right-hand side count (n = 64 beside n = 1, r = 14000: 14 MB a slot)
+        if (c >= CLS_ROW && d.F > 0)
+            P.slotr_bytes[c - CLS_ROW] = std::max(P.slotr_bytes[c - CLS_ROW], srom::lu64_slot_bytes(d.n, d.r));
     }
     long long all_items = 0;
     for (int c = 0; c < NCLS; ++c) all_items += P.n_items[c];
@@ -556,7 +560,6 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
         if (P.n_items[CLS_ROW + q] == 0) continue;
         P.gridr[q] = std::min<long long>(P.n_items[CLS_ROW + q],
                                          (long long)srom::lu64_blocks_per_sm(row_threads(q), P.r_nmax[q]) * h->sm_count);
-        P.slotr_bytes[q] = srom::lu64_slot_bytes(P.r_nmax[q], P.r_rmax[q]);
         P.need_scratch = true;
     }
     if (P.n_items[1] > 0) {
