@@ -63,7 +63,10 @@ typedef struct {
                               systems up to n = 512 (larger ones use the SROM_MIXED_FP32 kernel) */
 #define SROM_MIXED_AUTO 3  /* each system on the faster of the two mixed kernels for its order and
                               right-hand sides: as srom_tune measured, else the tensor-core kernel
-                              from n = 320 to 512 and the CUDA-core kernel elsewhere            */
+                              from n = 320 to 512 and the CUDA-core kernel elsewhere.  In a call with
+                              more systems of orders up to 320 than multiprocessors these are solved
+                              in FP64 outright (steps = 0), which is faster there (not with
+                              SROM_FLAG_MIXED_EVERY)                                            */
 
 /* ---- sweep flags ---------------------------------------------------------------------- */
 #define SROM_FLAG_FALLBACK_FP64 1 /* re-solve non-converged frequencies in FP64 (steps = -1);

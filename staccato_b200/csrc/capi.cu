@@ -444,6 +444,15 @@ int mixed_class(const srom_handle *h, int n, int r, int flags) {
 // depends on r, and srom_tune measures it.
 constexpr int TC_AUTO_MIN_N = 320;
 
+// SROM_MIXED_AUTO: a call of more systems than multiprocessors solves orders up to this one in FP64 outright
+// (steps = 0).  The row kernel holds two to six such systems a multiprocessor (one from n = 257), the mixed
+// kernels one.  592 systems, r = 4, well conditioned (one correction), FP64 against the faster mixed kernel:
+// n = 96 0.30 / 0.66 ms; 128 0.51 / 0.99; 200 1.49 / 2.19; 256 2.60 / 2.98; 300 4.32 / 4.75; 330 5.44 / 5.67 (r = 1
+// 5.30 / 5.23); 384 7.77 / 6.99; 220 systems: n = 96 0.22 / 0.35 ms; 200 0.72 / 1.08; 300 2.11 / 2.34.  With up to a
+// system a multiprocessor it is even or up to 18 % slower (148 systems: n = 128 0.28 / 0.26 ms; 256 0.88 / 0.77).
+// A batch of 16 models, orders 24 to 512: 117.4 -> 105.4 ms.
+constexpr int FP64_AUTO_MAX_N = 320;
+
 // Whether a mixed system of the global class runs on the tensor-core kernel.
 bool use_tc(const srom_handle *h, int n, int r, int precision) {
     if (n > srom::TC_MAX_N) return false;
@@ -504,6 +513,18 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
             }
         if (big < 0 || srom::global_panel_fits(gn, gr, h->max_smem_optin)) break;
         cls[big] = 2;
+    }
+    // SROM_MIXED_AUTO: the orders on which FP64 is the faster form once the call fills the GPU (an order that
+    // srom_tune measured against it stays where that put it)
+    if (o.precision == SROM_MIXED_AUTO && !(o.flags & SROM_FLAG_MIXED_EVERY)) {
+        auto outright = [&](int i) {
+            return cls[i] == 1 && roms[i].n <= FP64_AUTO_MAX_N && !h->tune_mixed.count(((long long)roms[i].n << 16) | roms[i].r);
+        };
+        long long items = 0;
+        for (int i = 0; i < n_roms; ++i)
+            if (outright(i)) items += roms[i].F;
+        for (int i = 0; i < n_roms; ++i)
+            if (items > h->sm_count && outright(i)) cls[i] = 0;
     }
     // mixed systems of the global class that the tensor-core kernel takes (SROM_MIXED_TC: every
     // one it can; SROM_MIXED_AUTO: where it is the faster); if the kernel cannot run their
