@@ -50,7 +50,14 @@ __global__ void transpose_kernel(const double *__restrict__ V, int64_t N, int k,
 // staged 32 entries at a time in the warp's shared-memory slot (coalesced loads), so that
 // the Vt gathers of SPMM_DEPTH consecutive entries are independent loads in flight together.
 // Every Y entry is the sequential FMA chain over the row's entries in storage order.
-constexpr int SPMM_THREADS = 256;
+//
+// CTAs of four warps, a warp a node, more of them than are resident: the hardware hands out the next CTA as one
+// ends.  With one resident wave that strides over the nodes, the long rows (a vertex node couples to 195 columns,
+// the average to 80) fell to the same warps whenever the wave's length met a multiple of a mesh layer's.  Two
+// matrices, 96 columns: 30,927 rows 160 -> 96 us, 41,175 rows 160 -> 121 us, 107,163 rows 316 -> 277 us; CTAs of
+// eight warps 113 / 141 / 326 us, of two 99 / 125 / 282 us.
+constexpr int SPMM_THREADS = 128;
+constexpr int SPMM_MMA_CTAS = 4;  // resident CTAs an SM of spmm_mma_kernel (128 registers a thread)
 constexpr int SPMM_WARPS = SPMM_THREADS / 32;
 constexpr int SPMM_DEPTH = 4;
 
@@ -165,7 +172,7 @@ __device__ __forceinline__ bool same_columns(int64_t r0, const int64_t *__restri
 // fall in four lines).  Tet10 block: 0.20 -> 0.14 ms at k = 32, 0.22 -> 0.20 ms at k = 48.  One or three
 // matrices would fill three or nine rows of the eight: spmm_full_kernel.
 template <int TP>
-__global__ void __launch_bounds__(SPMM_THREADS, 2) spmm_mma_kernel(int64_t N, const int64_t *__restrict__ rowptr,
+__global__ void __launch_bounds__(SPMM_THREADS, SPMM_MMA_CTAS) spmm_mma_kernel(int64_t N, const int64_t *__restrict__ rowptr,
                                                                    const int *__restrict__ colind, int base,
                                                                    ProjVals vals, const double *__restrict__ Vt0, int k,
                                                                    int ldv, double *__restrict__ Y0, int ldy,
@@ -278,36 +285,34 @@ __global__ void __launch_bounds__(SPMM_THREADS) spmm_full_kernel(int64_t N, cons
     }
 }
 
-// grid = at most one wave of resident CTAs (the row loop is grid-strided)
+// wave: at most one wave of resident CTAs (the node loop is grid-strided), else a warp a node
 template <int CPL, int NMAT>
-static void spmm_full_launch(int grid, cudaStream_t st, int64_t N, const int64_t *rowptr, const int *colind,
+static void spmm_full_launch(int grid, bool wave, cudaStream_t st, int64_t N, const int64_t *rowptr, const int *colind,
                              int base, const ProjVals &vals, const double *Vt, int k, int ldv, double *Y, int ldy,
-                             int64_t y_stride) {
-    int per_sm = 0, dev = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmm_full_kernel<CPL, NMAT>, SPMM_THREADS, 0) ==
-            cudaSuccess &&
-        cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && per_sm > 0)
+                             int64_t y_stride, int sms) {
+    int per_sm = 0;
+    if (wave && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmm_full_kernel<CPL, NMAT>, SPMM_THREADS, 0) ==
+                    cudaSuccess && per_sm > 0)
         grid = std::min(grid, per_sm * sms);
     spmm_full_kernel<CPL, NMAT><<<grid, SPMM_THREADS, 0, st>>>(N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy,
                                                                y_stride);
 }
 
 template <int TP>
-static void spmm_mma_launch(int grid, cudaStream_t st, int64_t N, const int64_t *rowptr, const int *colind, int base,
-                            const ProjVals &vals, const double *Vt, int k, int ldv, double *Y, int ldy, int64_t y_stride,
-                            int sms) {
-    spmm_mma_kernel<TP><<<std::min(grid, 2 * sms), SPMM_THREADS, 0, st>>>(N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy,
-                                                                         y_stride);
+static void spmm_mma_launch(int grid, bool wave, cudaStream_t st, int64_t N, const int64_t *rowptr, const int *colind,
+                            int base, const ProjVals &vals, const double *Vt, int k, int ldv, double *Y, int ldy,
+                            int64_t y_stride, int sms) {
+    if (wave) grid = std::min(grid, SPMM_MMA_CTAS * sms);
+    spmm_mma_kernel<TP><<<grid, SPMM_THREADS, 0, st>>>(N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride);
 }
 
 template <int CPL>
-static void launch_spmm_full(int grid, cudaStream_t st, int64_t N, const int64_t *rowptr, const int *colind,
+static void launch_spmm_full(int grid, bool wave, cudaStream_t st, int64_t N, const int64_t *rowptr, const int *colind,
                              int base, const ProjVals &vals, int n_mats, const double *Vt, int k, int ldv, double *Y,
-                             int ldy, int64_t y_stride) {
-    if (n_mats == 1) spmm_full_launch<CPL, 1>(grid, st, N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride);
-    else if (n_mats == 2) spmm_full_launch<CPL, 2>(grid, st, N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride);
-    else spmm_full_launch<CPL, 3>(grid, st, N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride);
+                             int ldy, int64_t y_stride, int sms) {
+    if (n_mats == 1) spmm_full_launch<CPL, 1>(grid, wave, st, N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride, sms);
+    else if (n_mats == 2) spmm_full_launch<CPL, 2>(grid, wave, st, N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride, sms);
+    else spmm_full_launch<CPL, 3>(grid, wave, st, N, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride, sms);
 }
 
 // Upper-triangle storage of a symmetric matrix (the reference's CSR,
@@ -858,27 +863,31 @@ cudaError_t launch_spmm(int64_t N, const int64_t *rowptr, const int *colind, int
                         int n_mats, const double *Vt, int k, double *Y, int64_t y_stride, int sms, cudaStream_t st) {
     const int threads = SPMM_THREADS;
     const int64_t warps_needed = (N + 2) / 3;
-    int grid = (int)std::min<int64_t>((warps_needed * 32 + threads - 1) / threads, (int64_t)sms * 8);
+    const int grid = (int)std::min<int64_t>((warps_needed * 32 + threads - 1) / threads, 1 << 30);
     // window by window (PRJ_WIN columns of the basis at a time), each into its columns of Y
     for (int j0 = 0; j0 < k; j0 += PRJ_WIN) {
         const int kw = std::min(PRJ_WIN, k - j0);
         const double *Vw = Vt + j0;
         double *Yw = Y + j0;
+        // Narrow windows of many nodes have little work a CTA and average out in one wave: 107,163 rows, a CTA a
+        // four nodes against one wave: k = 32 166 / 149 us (one matrix), 152 / 141 (two), 262 / 252 (three), k = 64 236 /
+        // 225 (two; one matrix 158 / 196).  At 41,175 rows k = 32 takes 58 / 66 us, 67 / 76 and 115 / 149.
+        const bool wave = (kw <= 32 || (n_mats == 2 && kw <= 64)) && warps_needed > (int64_t)160 * sms;
         // two matrices, even rows (the window starts on a multiple of 128 columns), up to 48 columns: the tensor
         // cores.  Beyond, a node's gathers no longer fit one warp's registers and its values and columns are read
         // once a 48-column part (Tet10 block: 0.20 against 0.22 ms at 48 columns, 0.26 against 0.22 at 64)
         if (n_mats == 2 && kw <= 48 && (k & 1) == 0 && (y_stride & 1) == 0) {
             auto go = kw <= 32 ? spmm_mma_launch<2> : spmm_mma_launch<3>;
-            go(grid, st, N, rowptr, colind, base, vals, Vw, kw, k, Yw, k, y_stride, sms);
-        } else if (kw <= 32) launch_spmm_full<1>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
-        else if (kw <= 64) launch_spmm_full<2>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
-        else if (kw <= 96) launch_spmm_full<3>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
-        else launch_spmm_full<4>(grid, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride);
+            go(grid, wave, st, N, rowptr, colind, base, vals, Vw, kw, k, Yw, k, y_stride, sms);
+        } else if (kw <= 32) launch_spmm_full<1>(grid, wave, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride, sms);
+        else if (kw <= 64) launch_spmm_full<2>(grid, wave, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride, sms);
+        else if (kw <= 96) launch_spmm_full<3>(grid, wave, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride, sms);
+        else launch_spmm_full<4>(grid, wave, st, N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k, y_stride, sms);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (upper) {
-            spmm_upper_mirror_kernel<<<grid, threads, 0, st>>>(N, rowptr, colind, base, vals, n_mats, Vw, kw, k, Yw, k,
-                                                               y_stride);
+            spmm_upper_mirror_kernel<<<std::min(grid, 16 * sms), threads, 0, st>>>(N, rowptr, colind, base, vals, n_mats, Vw, kw, k,
+                                                                                   Yw, k, y_stride);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
