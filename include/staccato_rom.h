@@ -74,7 +74,7 @@ typedef struct {
                                      contraction shows tol cannot be reached in max_refine */
 #define SROM_FLAG_KEEP_FACTORS 2  /* write LU factors + pivots into desc.LU / desc.ipiv (FP64) */
 #define SROM_FLAG_MIXED_EVERY 4   /* mixed forms: factor every system in FP32.  Without it, systems
-                                     small enough for two FP64 shared-memory factorisations per SM
+                                     of which two fit an SM's shared memory in FP64
                                      (n <= ~84) are solved by the FP64 kernel outright (steps = 0),
                                      which is faster than FP32 factors plus refinement there   */
 
