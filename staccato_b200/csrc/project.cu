@@ -894,12 +894,28 @@ cudaError_t launch_spmm(int64_t N, const int64_t *rowptr, const int *colind, int
     return cudaSuccess;
 }
 
-// matrices per launch: 24 warps at most (768 threads, <= 85 registers a thread) for windows
-// up to 12 tiles wide, 16 warps (512 threads) for wider ones
-static int vty_group(int ka, int kb, int n_mats) {
-    const int nband = ((ka + 7) & ~7) / 8, ntile = ((kb + 7) & ~7) / 8;
-    return std::max(1, std::min(n_mats, (ntile > 12 ? 16 : 24) / nband));
+// Matrices per launch of vty_partial_kernel: a matrix takes two warps a pair of 8-row bands, and a launch at most
+// 24 warps (768 threads, <= 85 registers a thread) for windows up to 12 tiles wide, 16 (512) for wider ones.
+constexpr int vty_warps(int nband) { return 2 * ((nband + 1) / 2); }
+constexpr int vty_max_warps(int ntile) { return ntile > 12 ? 16 : 24; }
+constexpr int vty_group(int nband, int ntile, int n_mats) {
+    return std::max(1, std::min(n_mats, vty_max_warps(ntile) / vty_warps(nband)));
 }
+constexpr size_t vty_smem(int nband, int ntile, int nm) {  // two chunks of 32 rows, leading dimensions padded by 4
+    return sizeof(double) * (size_t)2 * 32 * ((8 * nband + 4) + (size_t)nm * (8 * ntile + 4));
+}
+// every window and matrix count: the launch's threads within its bound, its shared memory within a CTA's 227 KB
+constexpr bool vty_fits() {
+    for (int nband = 1; nband <= PRJ_WIN / 8; ++nband)
+        for (int ntile = 1; ntile <= PRJ_WIN / 8; ++ntile)
+            for (int n_mats = 1; n_mats <= PRJ_MAX_MATS; ++n_mats) {
+                const int nm = vty_group(nband, ntile, n_mats);
+                if (nm * vty_warps(nband) > vty_max_warps(ntile) || vty_smem(nband, ntile, nm) > (size_t)227 * 1024)
+                    return false;
+            }
+    return true;
+}
+static_assert(vty_fits(), "vty_partial_kernel's launches fit their bounds");
 
 size_t vty_partial_doubles(int k, int n_mats, int nblk) {
     const int kp = (std::min(k, PRJ_WIN) + 7) & ~7;
@@ -908,9 +924,9 @@ size_t vty_partial_doubles(int k, int n_mats, int nblk) {
 
 template <int TH, int MAXT>
 static cudaError_t vty_launch(int64_t N, const VtyWindow &w, int nm, int nblk, double *partial, cudaStream_t st) {
-    const int kap = (w.ka + 7) & ~7, kbp = (w.kb + 7) & ~7;
-    const int threads = 32 * nm * 2 * ((kap / 8 + 1) / 2);
-    const size_t smem = sizeof(double) * (size_t)2 * 32 * ((kap + 4) + (size_t)nm * (kbp + 4));
+    const int nband = (w.ka + 7) / 8, ntile = (w.kb + 7) / 8;
+    const int threads = 32 * nm * vty_warps(nband);
+    const size_t smem = vty_smem(nband, ntile, nm);
     // rows of even length: every row of Vt and Y starts on 16 bytes
     const bool pairs = ((w.ldv | w.ldy | w.ka | w.kb) & 1) == 0 && (w.y_stride & 1) == 0 &&
                        ((reinterpret_cast<uintptr_t>(w.Vt) | reinterpret_cast<uintptr_t>(w.Y)) & 15) == 0;
@@ -933,16 +949,16 @@ cudaError_t launch_vty(int64_t N, int k, const double *Vt, const double *Y, int6
         for (int j0 = 0; j0 < k; j0 += PRJ_WIN) {
             const int kb = std::min(PRJ_WIN, k - j0);
             const int kbp = (kb + 7) & ~7, ntile = kbp / 8;
-            const int group = vty_group(ka, kb, n_mats);
+            const int group = vty_group(kap / 8, ntile, n_mats);
             for (int m0 = 0; m0 < n_mats; m0 += group) {
                 const int nm = std::min(group, n_mats - m0);
                 const VtyWindow w{Vt + i0, ka, k, Y + m0 * y_stride + j0, kb, k, y_stride};
                 double *Pm = partial + (int64_t)m0 * nblk * kap * kbp;
                 cudaError_t e;
-                if (ntile <= 4) e = vty_launch<2, 768>(N, w, nm, nblk, Pm, st);
-                else if (ntile <= 8) e = vty_launch<4, 768>(N, w, nm, nblk, Pm, st);
-                else if (ntile <= 12) e = vty_launch<6, 768>(N, w, nm, nblk, Pm, st);
-                else e = vty_launch<8, 512>(N, w, nm, nblk, Pm, st);
+                if (ntile <= 4) e = vty_launch<2, 32 * vty_max_warps(4)>(N, w, nm, nblk, Pm, st);
+                else if (ntile <= 8) e = vty_launch<4, 32 * vty_max_warps(8)>(N, w, nm, nblk, Pm, st);
+                else if (ntile <= 12) e = vty_launch<6, 32 * vty_max_warps(12)>(N, w, nm, nblk, Pm, st);
+                else e = vty_launch<8, 32 * vty_max_warps(16)>(N, w, nm, nblk, Pm, st);
                 if (e != cudaSuccess) return e;
             }
             ProjOut o{};

@@ -52,6 +52,14 @@ def test_projection_tiles(handle, nodes, extra, k, mats):
         assert (np.abs(r.cpu().numpy() - ref) <= 4 * n * np.finfo(float).eps * scale).all()
 
 
+# last windows of every number of 8-column bands after a full 128-column one (three matrices and five bands, k = 161 to
+# 168, took more threads than the kernel may have)
+@pytest.mark.parametrize("mats,k", [(3, 129), (3, 144), (3, 152), (3, 160), (3, 161), (3, 165), (3, 168), (3, 169), (3, 184),
+                                    (3, 200), (3, 216), (3, 232), (3, 248), (3, 256), (3, 293), (2, 165), (1, 165)])
+def test_projection_windows(handle, mats, k):
+    test_projection_tiles(handle, 37, 2, k, mats)
+
+
 @pytest.mark.parametrize("n,k,passes", [(5, 5, 2), (33, 7, 2), (64, 32, 2), (127, 33, 2), (1001, 40, 3), (4096, 96, 2),
                                         (2000, 129, 2), (3333, 200, 2)])
 def test_orthonormalize_tiles(handle, n, k, passes):
