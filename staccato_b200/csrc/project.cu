@@ -13,6 +13,7 @@
 // (mma.sync m8n8k4 f64): each CTA reduces a contiguous row range into a private k x k
 // partial, and a second kernel sums the partials in CTA order (deterministic).
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 
 #include "project_kernels.h"
@@ -666,9 +667,13 @@ __global__ void __launch_bounds__(GS_CT) gs_chol_kernel(const double *__restrict
         for (int i = 0; i < GS_B; ++i) x[i] = i == c && c < b ? 1.0 : 0.0;
 #pragma unroll
         for (int l = GS_B - 1; l >= 0; --l) {
-            x[l] *= rd[l];
+            // rows below the diagonal stay out: at a pivot that broke down (a column dependent on those before it)
+            // rd[l] and G[.][l] are not finite, and 0 times them would spread to the columns before
+            if (l <= c) {
+                x[l] *= rd[l];
 #pragma unroll
-            for (int i = 0; i < l; ++i) x[i] = fma(-G[i][l], x[l], x[i]);
+                for (int i = 0; i < l; ++i) x[i] = fma(-G[i][l], x[l], x[i]);
+            }
         }
 #pragma unroll
         for (int i = 0; i < GS_B; ++i) rinv[i * GS_B + c] = i <= c ? x[i] : 0.0;
@@ -729,6 +734,7 @@ __global__ void __launch_bounds__(32 * GS_UW, 3) gs_update_kernel(double *__rest
     }
     __syncthreads();
     double *T = Hs + warp * 16 * GS_LDB;
+    bool finite = true;
 #pragma unroll
     for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -736,9 +742,24 @@ __global__ void __launch_bounds__(32 * GS_UW, 3) gs_update_kernel(double *__rest
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 T[(8 * x + lr) * GS_LDB + 8 * t + 2 * lk + h] = acc[x][t][h];
+                finite = finite && fabs(acc[x][t][h]) <= DBL_MAX;
                 acc[x][t][h] = 0.0;
             }
+    finite = __all_sync(0xffffffffu, finite);
     __syncwarp();
+    if (!finite) {
+        // a column that broke down in the pass before, or came in not finite: the zeros below Rinv's diagonal would
+        // carry it into the columns before it in the same 8-column tile, so these sums end at the diagonal
+#pragma unroll 1
+        for (int e = lane; e < 16 * b; e += 32) {
+            const int row = e & 15, c = e >> 4;
+            double s = 0.0;
+#pragma unroll 1
+            for (int k = 0; k <= c; ++k) s = fma(T[row * GS_LDB + k], Rs[k * GS_LDB + c], s);
+            if (r0 + row < N) V[r0 + row + (int64_t)(j0 + c) * ldv] = s;
+        }
+        return;
+    }
 #pragma unroll
     for (int k = 0; k < GS_B; k += 4) {
         double p[2];

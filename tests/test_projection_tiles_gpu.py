@@ -74,3 +74,24 @@ def test_orthonormalize_tiles(handle, n, k, passes):
     q, r = np.linalg.qr(V)
     q = q * np.sign(np.diag(r))
     assert np.abs(Q - q).max() <= 1e-12 * np.linalg.cond(V)
+
+
+# a zero column in a panel: it and the panel's later columns come out non-finite, the columns before it are untouched
+@pytest.mark.parametrize("n,k,zero", [(500, 32, 20), (500, 32, 31), (777, 30, 1), (300, 17, 16), (1000, 70, 52), (4000, 96, 95),
+                                      (640, 64, 33)])
+def test_orthonormalize_keeps_the_columns_before_a_dependent_one(handle, n, k, zero):
+    import torch
+
+    rng = np.random.default_rng(zero)
+    V = rng.standard_normal((n, k)) + 0.3 * rng.standard_normal((n, 1))
+    V[:, zero] = 0.0
+    Vd = torch.from_numpy(np.ascontiguousarray(V.T)).cuda()
+    orthonormalize(handle, Vd, 2)
+    Q = Vd.cpu().numpy().T
+    assert not np.isfinite(Q[:, zero]).any()
+    Q = Q[:, :zero]
+    assert np.isfinite(Q).all()
+    assert np.abs(Q.T @ Q - np.eye(zero)).max() <= 1e-13 * max(1.0, k / 32)
+    q, r = np.linalg.qr(V[:, :zero])
+    q = q * np.sign(np.diag(r))
+    assert np.abs(Q - q).max() <= 1e-12 * np.linalg.cond(V[:, :zero])
