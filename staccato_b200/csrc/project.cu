@@ -641,7 +641,8 @@ __global__ void __launch_bounds__(GS_CT) gs_chol_kernel(const double *__restrict
     __syncthreads();
     // G = L D L^T by rows: row j is final before step j, and R[j][c] = G[j][c] / sqrt(G[j][j])
     for (int j = 0; j + 1 < b; ++j) {
-        const double t = G[j][c] * __drcp_rn(G[j][j]);
+        // (columns of norm below about 1e-154: the reciprocal of their pivot overflows)
+        const double d = G[j][j], t = d < 0x1p-1000 ? G[j][c] / d : G[j][c] * __drcp_rn(d);
 #pragma unroll
         for (int q = 0; q < GS_CR; ++q) {
             const int a = a0 + 8 * q;

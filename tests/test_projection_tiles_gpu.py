@@ -95,3 +95,22 @@ def test_orthonormalize_keeps_the_columns_before_a_dependent_one(handle, n, k, z
     q, r = np.linalg.qr(V[:, :zero])
     q = q * np.sign(np.diag(r))
     assert np.abs(Q - q).max() <= 1e-12 * np.linalg.cond(V[:, :zero])
+
+
+# columns of very small and very large norm: their squares stay in range, the reciprocals of the squares need not
+@pytest.mark.parametrize("scale", [1e-157, 1e-155, 1e-150, 1e150])
+def test_orthonormalize_range(handle, scale):
+    import torch
+
+    rng = np.random.default_rng(7)
+    n, k = 900, 40
+    V = rng.standard_normal((n, k)) + 0.3 * rng.standard_normal((n, 1))
+    Vd = torch.from_numpy(np.ascontiguousarray(scale * V.T)).cuda()
+    orthonormalize(handle, Vd, 2)
+    Q = Vd.cpu().numpy().T
+    assert np.abs(Q.T @ Q - np.eye(k)).max() <= 1e-13 * max(1.0, k / 32)
+    q, r = np.linalg.qr(V)
+    q = q * np.sign(np.diag(r))
+    # the first pass works on squares that have lost digits at 1e-157 (subnormal, n scale^2 = 9e-312: 5e-13 of one)
+    tol = 1e-12 if scale > 1e-154 else 1e-12 + 900 * 2.0 ** -1074 / scale ** 2
+    assert np.abs(Q - q).max() <= tol * np.linalg.cond(V)
