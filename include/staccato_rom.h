@@ -175,13 +175,15 @@ SROM_API int srom_graph_destroy(srom_graph *graph);
 /*
  * Autotune the kernel choices for each order in n_values with r right-hand sides, timed on a
  * synthetic system (2 x SMs frequencies) and used by later sweeps on this handle:
- *   - FP64: the whole system in shared memory vs. the blocked LU in global scratch;
- *   - mixed forms, where the FP64 choice is the shared-memory kernel: solving such systems in
- *     FP64 outright (steps = 0) vs. complex-FP32 factors in the mixed global kernel plus
- *     refinement (without a measurement the rule is: FP64 when two systems fit an SM).
+ *   - FP64, orders whose system fits shared memory (n <= ~112): a thread a row or the next larger thread count;
+ *   - mixed forms, the same orders: solving such systems in FP64 outright (steps = 0) vs.
+ *     complex-FP32 factors in the mixed global kernel plus refinement (without a measurement the
+ *     rule is: FP64 when two systems fit an SM's shared memory);
+ *   - SROM_MIXED_AUTO, orders 96 to 512: the CUDA-core or the tensor-core mixed kernel.
  * Panel width, tile shapes and threads per system are fixed per kernel by its register and
  * shared-memory budget (compile-time).  cache_path (or NULL) is a JSON file of earlier choices
- * for this device, read first and rewritten with new entries.
+ * for this device, read first and rewritten with new entries; a file of an earlier format (the choices of kernels
+ * that are gone) is not read and its entries are measured anew.
  */
 SROM_API int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char *cache_path);
 

@@ -66,10 +66,11 @@ struct srom_handle {
     };
     bool prof = false;
     std::vector<ProfRec> recs;
-    // FP64 storage class chosen by srom_tune per (n << 16 | r): 0 smem kernel, 1 global kernel
-    std::map<long long, int> tune_fp64;
-    // mixed-form routing chosen by srom_tune per (n << 16 | r) where the FP64 smem kernel is
-    // the FP64 choice: 0 solve in FP64 outright, 1 mixed global kernel
+    // threads a system of the FP64 row kernel chosen by srom_tune per (n << 16 | r), for the orders whose system fits
+    // shared memory: 0 the smallest count with a thread a row, 1 the next one up
+    std::map<long long, int> tune_wide;
+    // mixed-form routing of those orders chosen by srom_tune per (n << 16 | r): 0 solve in FP64 outright, 1 mixed
+    // global kernel
     std::map<long long, int> tune_mixed;
     // SROM_MIXED_AUTO's kernel chosen by srom_tune per (n << 16 | r): 0 CUDA-core, 1 tensor-core
     std::map<long long, int> tune_tc;
@@ -401,16 +402,11 @@ void patch_null_m(SweepPlan &P, const void *zero) {
 // less for more right-hand sides; every n > 768) run on the large-order FP64 kernel (class 2).
 bool large_order(const srom_handle *h, int n, int r) { return !srom::global_panel_fits(n, r, h->max_smem_optin); }
 
-// FP64 storage class of an n x n system with r right-hand sides: 0 smem kernel, 1 global
-// kernel, 2 large-order global kernel.  The tuning table (srom_tune) overrides the default
-// "smem when it fits".
+// FP64 storage class of an n x n system with r right-hand sides: 0 the whole system fits shared
+// memory, 2 large orders, 1 between.
 int fp64_class(const srom_handle *h, int n, int r) {
     if (large_order(h, n, r)) return 2;
-    const bool fits = srom::fp64_smem_bytes(n, r) <= (size_t)h->max_smem_optin;
-    if (!fits) return 1;
-    auto it = h->tune_fp64.find(((long long)n << 16) | r);
-    if (it != h->tune_fp64.end()) return it->second;
-    return 0;
+    return srom::fp64_smem_bytes(n, r) <= (size_t)h->max_smem_optin ? 0 : 1;
 }
 
 // Thread counts of the FP64 row kernel's classes: the smallest with a thread a row (wide: the next
@@ -420,6 +416,10 @@ int row_class(int n, bool wide) {
     int q = 0;
     while (row_threads(q) < n) ++q;
     return std::min(q + (wide ? 1 : 0), N_ROW - 1);
+}
+bool tuned_wide(const srom_handle *h, int n, int r) {
+    auto it = h->tune_wide.find(((long long)n << 16) | r);
+    return it != h->tune_wide.end() && it->second != 0;
 }
 
 // Mixed-form class: a system of which two fit an SM's shared memory in FP64 is solved by the FP64 row
@@ -482,10 +482,7 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
     }
     P.mixed = mixed;
     P.o = o;
-    // FP64: systems that fit shared memory use the smem kernel (unless tuned otherwise),
-    // the rest the global kernel.  Mixed: the smallest systems use the FP64 smem kernel
-    // (mixed_class), the rest the mixed global kernel.
-    const size_t smem_cap = (size_t)h->max_smem_optin;
+    // Mixed: the smallest systems are solved in FP64 outright (mixed_class), the rest by a mixed kernel.
     std::vector<RomDev> dev(n_roms);
     std::vector<int> cls(n_roms, -1);
     for (int i = 0; i < n_roms; ++i) {
@@ -548,18 +545,17 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
     if (P.b_nmax > srom::BIG_MAX_N)
         return set_err(h, SROM_ERR_UNSUPPORTED, "n=%d exceeds the largest supported order %d", P.b_nmax,
                        srom::BIG_MAX_N);
-    if (P.b_nmax > 0 && srom::global_smem_bytes(P.b_nmax, P.b_rmax, true) + srom::GLOBAL_STATIC_SMEM > smem_cap)
+    if (P.b_nmax > 0 && srom::global_smem_bytes(P.b_nmax, P.b_rmax, true) + srom::GLOBAL_STATIC_SMEM > (size_t)h->max_smem_optin)
         return set_err(h, SROM_ERR_UNSUPPORTED,
                        "n=%d with r=%d: the right-hand sides (n*r*16 bytes) exceed shared memory", P.b_nmax,
                        P.b_rmax);
-    // FP64 systems of orders up to 512 run on the row kernel; a measured "global" choice of
-    // srom_tune gives such a system the next larger thread count
+    // FP64 systems of orders up to 512 run on the row kernel, with the thread count that srom_tune measured, if any
     P.b_nmax = P.b_rmax = 0;
     for (int i = 0; i < n_roms; ++i) {
         const srom_rom_desc &d = roms[i];
         if (cls[i] < 0) continue;
         if (d.n <= srom::LU64_MAX_N && (cls[i] == 0 || cls[i] == 2 || (cls[i] == 1 && !mixed)))
-            cls[i] = CLS_ROW + row_class(d.n, cls[i] == 1 && srom::fp64_smem_bytes(d.n, d.r) <= smem_cap);
+            cls[i] = CLS_ROW + row_class(d.n, tuned_wide(h, d.n, d.r));
         P.keep = P.keep || d.LU;
         const int c = cls[i];
         int *nm = c == 1 ? &P.g_nmax : c == 2 ? &P.b_nmax : c == 3 ? &P.t_nmax : &P.r_nmax[c - CLS_ROW];
@@ -1421,6 +1417,7 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
     h->err.clear();
     if (count < 0 || (count > 0 && !n_values) || r < 1) return set_err(h, SROM_ERR_INVALID, "bad tuning request");
     DeviceGuard g(h->device);
+    constexpr int TUNE_FORMAT = 2;  // of the cache file; a new one for every change of what its choices mean
     cudaDeviceProp prop;
     SROM_CUDA(h, cudaGetDeviceProperties(&prop, h->device));
     // 1) cached choices for this device
@@ -1428,13 +1425,16 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
         if (FILE *fp = fopen(cache_path, "r")) {
             char line[512], dev[256] = {0};
             bool same_dev = false;
+            int format = 1;  // a file without the entry was measured on earlier kernels: its choices are measured anew
             while (fgets(line, sizeof line, fp)) {
-                if (sscanf(line, " \"device\": \"%255[^\"]\"", dev) == 1) same_dev = strcmp(dev, prop.name) == 0;
-                int n = 0, rr = 0;
+                sscanf(line, " \"format\": %d", &format);
+                if (sscanf(line, " \"device\": \"%255[^\"]\"", dev) == 1)
+                    same_dev = format == TUNE_FORMAT && strcmp(dev, prop.name) == 0;
+                int n = 0, rr = 0, threads = 0;
                 char kern[32] = {0};
-                if (same_dev && sscanf(line, " {\"precision\": \"fp64\", \"n\": %d, \"r\": %d, \"kernel\": \"%31[^\"]\"",
-                                       &n, &rr, kern) == 3)
-                    h->tune_fp64[((long long)n << 16) | rr] = strcmp(kern, "smem") == 0 ? 0 : 1;
+                if (same_dev && sscanf(line, " {\"precision\": \"fp64\", \"n\": %d, \"r\": %d, \"kernel\": \"smem\", \"threads\": %d",
+                                       &n, &rr, &threads) == 3 && n > 0 && n <= srom::LU64_MAX_N)
+                    h->tune_wide[((long long)n << 16) | rr] = threads > row_threads(row_class(n, false)) ? 1 : 0;
                 if (same_dev && sscanf(line, " {\"precision\": \"mixed\", \"n\": %d, \"r\": %d, \"kernel\": \"%31[^\"]\"",
                                        &n, &rr, kern) == 3)
                     h->tune_mixed[((long long)n << 16) | rr] = strcmp(kern, "fp64_smem") == 0 ? 0 : 1;
@@ -1445,9 +1445,9 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
             fclose(fp);
         }
     }
-    // 2) time both storage classes for every requested n that has no entry yet
+    // 2) time the choices of every requested n that has no entry yet
     struct Entry {
-        int n, r, cls;
+        int n, r, wide;  // -1: not measured
         float ms[2];
         int mcls;      // mixed routing (-1: not measured)
         float mms[2];  // mixed sweep: FP64 outright, mixed global kernel
@@ -1459,9 +1459,10 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
         const int n = n_values[q];
         if (n <= 0) continue;
         const long long key = ((long long)n << 16) | r;
-        // FP64: only a choice where the shared-memory kernel fits; the mixed kernels: orders
+        // FP64: two thread counts where the system fits shared memory; the mixed kernels: orders
         // from 96 up to the tensor-core kernel's limit
-        const bool need_fp64 = !h->tune_fp64.count(key) && srom::fp64_smem_bytes(n, r) <= (size_t)h->max_smem_optin;
+        const bool need_fp64 = (!h->tune_wide.count(key) || (r <= srom::MIXED_MAX_R && !h->tune_mixed.count(key))) &&
+                               srom::fp64_smem_bytes(n, r) <= (size_t)h->max_smem_optin;
         const bool need_tc = !h->tune_tc.count(key) && n >= 96 && n <= srom::TC_MAX_N && r <= srom::MIXED_MAX_R &&
                              srom::tc_supported(n, r, h->max_smem_optin, nullptr) &&
                              srom::global_panel_fits(n, r, h->max_smem_optin);
@@ -1525,12 +1526,12 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
         };
         const srom_sweep_opts o64{SROM_FP64, 5, 0.0, 0};
         for (int c = 0; c < 2 && rc == SROM_OK && need_fp64; ++c) {
-            h->tune_fp64[key] = c;
+            h->tune_wide[key] = c;
             rc = time_sweep(o64, &ent.ms[c]);
         }
         if (rc == SROM_OK && need_fp64) {
-            ent.cls = ent.ms[1] < ent.ms[0] ? 1 : 0;
-            h->tune_fp64[key] = ent.cls;
+            ent.wide = ent.ms[1] < ent.ms[0] ? 1 : 0;
+            h->tune_wide[key] = ent.wide;
         }
         // SROM_MIXED_AUTO's kernel: every system on the CUDA-core, then on the tensor-core kernel
         if (rc == SROM_OK && need_tc) {
@@ -1543,10 +1544,9 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
                 h->tune_tc[key] = ent.tcls;
             }
         }
-        // the mixed form's routing of such a system: the FP64 shared-memory kernel outright, or
-        // complex-FP32 factors in the mixed global kernel plus refinement (only a choice when the
-        // FP64 choice is the shared-memory kernel)
-        if (rc == SROM_OK && need_fp64 && ent.cls == 0 && r <= srom::MIXED_MAX_R) {
+        // the mixed form's routing of such a system: FP64 outright, or complex-FP32 factors in the mixed global
+        // kernel plus refinement
+        if (rc == SROM_OK && need_fp64 && r <= srom::MIXED_MAX_R) {
             const srom_sweep_opts om{SROM_MIXED_FP32, 5, 0.0, SROM_FLAG_FALLBACK_FP64};
             for (int c = 0; c < 2 && rc == SROM_OK; ++c) {
                 h->tune_mixed[key] = c;
@@ -1563,7 +1563,7 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
         cudaFree(buf);
         if (rc != SROM_OK) {
             if (need_fp64) {
-                h->tune_fp64.erase(key);
+                h->tune_wide.erase(key);
                 h->tune_mixed.erase(key);
             }
             if (need_tc) h->tune_tc.erase(key);
@@ -1575,19 +1575,19 @@ int srom_tune(srom_handle *h, const int *n_values, int count, int r, const char 
     if (cache_path && !measured.empty()) {
         FILE *fp = fopen(cache_path, "w");
         if (!fp) return set_err(h, SROM_ERR_INVALID, "cannot write %s", cache_path);
-        fprintf(fp, "{\n  \"device\": \"%s\",\n  \"entries\": [\n", prop.name);
-        const size_t total = h->tune_fp64.size() + h->tune_mixed.size() + h->tune_tc.size();
+        fprintf(fp, "{\n  \"format\": %d,\n  \"device\": \"%s\",\n  \"entries\": [\n", TUNE_FORMAT, prop.name);
+        const size_t total = h->tune_wide.size() + h->tune_mixed.size() + h->tune_tc.size();
         size_t k = 0;
-        for (const auto &kv : h->tune_fp64) {
+        for (const auto &kv : h->tune_wide) {
             const int n = (int)(kv.first >> 16), rr = (int)(kv.first & 0xffff);
             float ms0 = -1.f, ms1 = -1.f;
             for (const auto &m : measured)
-                if (m.n == n && m.r == rr && m.cls >= 0) {
+                if (m.n == n && m.r == rr && m.wide >= 0) {
                     ms0 = m.ms[0];
                     ms1 = m.ms[1];
                 }
-            fprintf(fp, "    {\"precision\": \"fp64\", \"n\": %d, \"r\": %d, \"kernel\": \"%s\", \"ms_smem\": %.4f, \"ms_global\": %.4f}%s\n",
-                    n, rr, kv.second == 0 ? "smem" : "global", ms0, ms1, ++k < total ? "," : "");
+            fprintf(fp, "    {\"precision\": \"fp64\", \"n\": %d, \"r\": %d, \"kernel\": \"smem\", \"threads\": %d, \"ms\": %.4f, \"ms_wide\": %.4f}%s\n",
+                    n, rr, row_threads(row_class(n, kv.second != 0)), ms0, ms1, ++k < total ? "," : "");
         }
         for (const auto &kv : h->tune_mixed) {
             const int n = (int)(kv.first >> 16), rr = (int)(kv.first & 0xffff);

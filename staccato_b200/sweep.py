@@ -260,7 +260,7 @@ class Graph:
 
 
 def tune(handle: _capi.Handle, n_values, r: int = 1, cache_path: Optional[str] = None) -> None:
-    """Autotune the FP64 kernel choice per order n (``srom_tune``), optionally with a JSON cache."""
+    """Autotune the kernel choices per order n (``srom_tune``), optionally with a JSON cache."""
     ns = (C.c_int * max(len(n_values), 1))(*[int(v) for v in n_values])
     check(handle.ptr, _capi.lib().srom_tune(handle.ptr, ns, len(n_values), int(r),
                                             None if cache_path is None else cache_path.encode()))
