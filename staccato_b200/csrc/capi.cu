@@ -361,8 +361,8 @@ namespace {
 
 // A validated, classified and ordered sweep: the host image of the device metadata
 // (descriptors, cost-ordered work lists, fallback list, zeroed counters) plus launch shapes.
-// Storage classes of a plan: 0 FP64 orders whose matrix fits shared memory (routed to the row
-// kernel), 1 FP64 above n = 512 or the CUDA-core mixed kernel, 2 FP64 of large orders (FP64 of both
+// Storage classes of a plan: 0 FP64 shared-memory kernel (first of all FP64 orders whose system fits
+// shared memory; most go on to the row kernel), 1 FP64 above n = 512 or the CUDA-core mixed kernel, 2 FP64 of large orders (FP64 of both
 // classes: sweep_large.cu), 3 tensor-core mixed kernel, 4..7 the FP64 row kernel (sweep_lu64.cu) with 64, 128, 256
 // and 512 threads a system.
 constexpr int NCLS = 8;
@@ -376,6 +376,8 @@ struct SweepPlan {
     size_t off_fb = 0, off_ctr = 0;
     long long n_items[NCLS] = {};
     double flops[NCLS] = {};
+    size_t smem_max = 0;           // class 0: the largest system's bytes
+    long long grid0 = 0;
     int g_nmax = 0, g_rmax = 0;    // class 1: the global kernels' largest order and RHS count
     int b_nmax = 0, b_rmax = 0;    // class 2: the large-order FP64 kernel's
     int t_nmax = 0, t_rmax = 0;    // class 3: the tensor-core kernel's
@@ -549,14 +551,48 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
         return set_err(h, SROM_ERR_UNSUPPORTED,
                        "n=%d with r=%d: the right-hand sides (n*r*16 bytes) exceed shared memory", P.b_nmax,
                        P.b_rmax);
-    // FP64 systems of orders up to 512 run on the row kernel, with the thread count that srom_tune measured, if any
+    // FP64 systems of orders up to 512 run on the row kernel, with the thread count that srom_tune measured, if any,
+    // except where the shared-memory kernel is the faster one.  In a call of up to a system a multiprocessor the two
+    // launches add up: its small systems run in the shadow of the larger ones on the row kernel, or, where it is those
+    // with many right-hand sides to a column that end last, all of them on the shared-memory kernel, if they fit it
+    // (100 systems of order 24, r = 200 and one of order 100: 0.32 ms together, 0.22 + 0.28 apart).
+    auto fp64_upto512 = [&](int i) {
+        return cls[i] >= 0 && roms[i].n <= srom::LU64_MAX_N && (cls[i] == 0 || cls[i] == 2 || (cls[i] == 1 && !mixed));
+    };
+    long long fp64_systems = 0;
+    for (int i = 0; i < n_roms; ++i)
+        if (fp64_upto512(i)) fp64_systems += roms[i].F;
+    auto small = [&](int i) {
+        return fp64_upto512(i) && srom::fp64_smem_faster(roms[i].n, roms[i].r, fp64_systems, h->sm_count) &&
+               srom::fp64_smem_bytes(roms[i].n, roms[i].r) + srom::GLOBAL_STATIC_SMEM <= (size_t)h->max_smem_optin;
+    };
+    const bool one_wave = fp64_systems <= h->sm_count;
+    bool row_needed = false, fit = true, tiny = true, wide = false;
+    for (int i = 0; i < n_roms; ++i)
+        if (fp64_upto512(i)) {
+            row_needed = row_needed || !small(i);
+            fit = fit && srom::fp64_smem_bytes(roms[i].n, roms[i].r) + srom::GLOBAL_STATIC_SMEM <= (size_t)h->max_smem_optin;
+            tiny = tiny && roms[i].n <= 32;
+        }
+    auto many_rhs = [&](int i) { return small(i) && roms[i].r >= 32 && roms[i].r > 4LL * roms[i].n; };
+    for (int i = 0; i < n_roms && one_wave && row_needed && fit; ++i)
+        wide = wide || many_rhs(i) || (tiny && small(i) && roms[i].r >= roms[i].n);
+    auto on_smem = [&](int i) {
+        return fp64_upto512(i) && (one_wave && row_needed ? wide || many_rhs(i) : small(i));
+    };
     P.b_nmax = P.b_rmax = 0;
     for (int i = 0; i < n_roms; ++i) {
         const srom_rom_desc &d = roms[i];
         if (cls[i] < 0) continue;
-        if (d.n <= srom::LU64_MAX_N && (cls[i] == 0 || cls[i] == 2 || (cls[i] == 1 && !mixed)))
-            cls[i] = CLS_ROW + row_class(d.n, tuned_wide(h, d.n, d.r));
         P.keep = P.keep || d.LU;
+        if (on_smem(i)) {
+            cls[i] = 0;
+            P.smem_max = std::max(P.smem_max, srom::fp64_smem_bytes(d.n, d.r));
+            P.n_items[0] += d.F;
+            P.flops[0] += lu_flops(d.n, d.r) * d.F;
+            continue;
+        }
+        if (fp64_upto512(i)) cls[i] = CLS_ROW + row_class(d.n, tuned_wide(h, d.n, d.r));
         const int c = cls[i];
         int *nm = c == 1 ? &P.g_nmax : c == 2 ? &P.b_nmax : c == 3 ? &P.t_nmax : &P.r_nmax[c - CLS_ROW];
         int *rm = c == 1 ? &P.g_rmax : c == 2 ? &P.b_rmax : c == 3 ? &P.t_rmax : &P.r_rmax[c - CLS_ROW];
@@ -572,6 +608,11 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
     long long all_items = 0;
     for (int c = 0; c < NCLS; ++c) all_items += P.n_items[c];
     if (all_items > INT32_MAX) return set_err(h, SROM_ERR_UNSUPPORTED, "too many systems");
+    if (P.n_items[0] > 0) {
+        const int bps = srom::fp64_smem_blocks_per_sm(P.smem_max);
+        if (bps <= 0) return set_err(h, SROM_ERR_UNSUPPORTED, "smem kernel cannot be resident (%zu B)", P.smem_max);
+        P.grid0 = std::min<long long>(P.n_items[0], (long long)bps * h->sm_count);
+    }
     for (int q = 0; q < N_ROW; ++q) {
         if (P.n_items[CLS_ROW + q] == 0) continue;
         P.gridr[q] = std::min<long long>(P.n_items[CLS_ROW + q],
@@ -641,7 +682,7 @@ size_t plan_scratch_bytes(const SweepPlan &P) {
 }
 
 // Counters live at off_ctr and must be zero when the launches start (the metadata copy zeroes
-// them, or zero_counters does): 1 global kernel, 2 fallback count, 3 fallback work, 4 tensor-core
+// them, or zero_counters does): 0 smem kernel, 1 global kernel, 2 fallback count, 3 fallback work, 4 tensor-core
 // error word, 6 tensor-core kernel, 8..11 row kernel.
 int enqueue_plan(srom_handle *h, const SweepPlan &P, char *dm, void *scratch, cudaStream_t st, bool zero_counters,
                  bool profile) {
@@ -668,6 +709,11 @@ int enqueue_plan(srom_handle *h, const SweepPlan &P, char *dm, void *scratch, cu
         ProfScope ps(h, q < 2 ? "fp64_smem" : "fp64_global", P.n_items[c], P.flops[c], 0.0);
         cudaError_t e = srom::launch_lu64(row_threads(q), a, (int)P.gridr[q], st);
         if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "fp64 row launch: %s", cudaGetErrorString(e));
+    }
+    if (rc == SROM_OK && P.n_items[0] > 0) {
+        ProfScope ps(h, "fp64_smem", P.n_items[0], P.flops[0], 0.0);
+        cudaError_t e = srom::launch_fp64_smem(d_roms, items(0), (int)P.n_items[0], d_ctr, P.smem_max, (int)P.grid0, st);
+        if (e != cudaSuccess) rc = set_err(h, SROM_ERR_CUDA, "fp64 smem launch: %s", cudaGetErrorString(e));
     }
     Item *fb_items = nullptr;
     int *fb_count = nullptr;

@@ -6,7 +6,7 @@
 // its possible failure at run time are not acceptable.  srom_sweep needs a handle, whose
 // creation and first calls allocate descriptor staging and one scratch matrix per resident
 // CTA; this entry point instead takes one ROM descriptor, uses the scratch array below, and
-// runs the same FP64 row kernel (bit-identical results).
+// runs the same FP64 kernels (bit-identical results).
 //
 // The scratch array lives for as long as the library is loaded, on every device that loads
 // it.  Every call uses the same array: its contents are whatever the last call left, so the
@@ -158,21 +158,27 @@ extern "C" int srom_sweep_fp64_noalloc(const srom_rom_desc *d, void *cuda_stream
     noalloc_prepare<<<(d->F + 255) / 256, 256, 0, st>>>(R, base);
     if ((e = cudaGetLastError()) != cudaSuccess)
         return fail(err, err_len, SROM_ERR_CUDA, "prepare launch", cudaGetErrorString(e));
-    int threads = 64;
-    while (threads < d->n) threads *= 2;
     srom::GlobalArgs a{};
     a.roms = reinterpret_cast<const srom::RomDev *>(base);
     a.items = reinterpret_cast<const srom::Item *>(base + NOALLOC_HDR_BYTES);
     a.n_items = d->F;
     a.counter = reinterpret_cast<int *>(base + 256);
-    a.scratch = base + NOALLOC_HDR_BYTES + NOALLOC_ITEM_BYTES;
-    a.slot_bytes = srom::lu64_slot_bytes(d->n, d->r);
-    a.n_max = d->n;
-    a.r_max = d->r;
-    const long long slots = (long long)(NOALLOC_SLOT_BYTES / (size_t)a.slot_bytes);
-    const long long grid =
-        std::min<long long>(std::min<long long>(d->F, (long long)sms * srom::lu64_blocks_per_sm(threads, d->n)), slots);
-    e = grid > 0 ? srom::launch_lu64(threads, a, (int)grid, st) : cudaErrorInvalidValue;
+    const size_t small = srom::fp64_smem_bytes(d->n, d->r);
+    if (srom::fp64_smem_faster(d->n, d->r, d->F, sms) && small + srom::GLOBAL_STATIC_SMEM <= (size_t)smem_optin) {
+        const long long grid = std::min<long long>(d->F, (long long)sms * srom::fp64_smem_blocks_per_sm(small));
+        e = grid > 0 ? srom::launch_fp64_smem(a.roms, a.items, d->F, a.counter, small, (int)grid, st) : cudaErrorInvalidValue;
+    } else {
+        int threads = 64;
+        while (threads < d->n) threads *= 2;
+        a.scratch = base + NOALLOC_HDR_BYTES + NOALLOC_ITEM_BYTES;
+        a.slot_bytes = srom::lu64_slot_bytes(d->n, d->r);
+        a.n_max = d->n;
+        a.r_max = d->r;
+        const long long slots = (long long)(NOALLOC_SLOT_BYTES / (size_t)a.slot_bytes);
+        const long long grid = std::min<long long>(
+            std::min<long long>(d->F, (long long)sms * srom::lu64_blocks_per_sm(threads, d->n)), slots);
+        e = grid > 0 ? srom::launch_lu64(threads, a, (int)grid, st) : cudaErrorInvalidValue;
+    }
     if (e != cudaSuccess) return fail(err, err_len, SROM_ERR_CUDA, "sweep launch", cudaGetErrorString(e));
     if (d->n_out > 0) {
         srom::BackProj b{d->n, d->r, d->F, d->n_out, d->ldc, reinterpret_cast<const double2 *>(d->C),

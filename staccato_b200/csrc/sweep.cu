@@ -11,7 +11,9 @@
 // unit-lower triangle for the U rows (warp shuffles), and update the remaining rows with
 // register-tiled complex FMAs.  No CTA barrier separates the column groups.  FP64 sweeps run on
 // sweep_lu64.cu (orders up to 512) and sweep_large.cu (above); the FP64 instances here re-solve the
-// mixed form's non-converged systems of orders above 512, whose number only the device knows.
+// mixed form's non-converged systems of orders above 512, whose number only the device knows, and, with
+// matrix and right-hand sides whole in shared memory, solve the smallest orders in FP64 where that is
+// the faster form (fp64_smem_faster).
 //
 // Precision forms
 //   FP64  (double2): reproduces LAPACK zgetrf/zgetrs as restated in the oracle bit for bit:
@@ -38,6 +40,83 @@
 #include "sweep_common.cuh"
 
 namespace srom {
+
+
+// ====================================================================================
+// smem class (FP64): the whole n x n matrix and the right-hand sides in shared memory, unblocked right-looking LU,
+// one warp searches each pivot.  Nothing passes through global memory between assembly and solution, and all 256
+// threads share the right-hand sides: a system of few columns, or of many right-hand sides to a column, is bound by
+// those latencies and not by the pivot chain that sweep_lu64.cu shortens (fp64_smem_faster has both sides' times).
+// ====================================================================================
+__device__ __forceinline__ void panel_factor_smem(double2 *P, int ldp, int m, int ncols, int *ipiv, int *s_info,
+                                  double2 *Bs, int ldbs, int nrhs, int *s_bc) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int jj = 0; jj < ncols; ++jj) {
+        if (warp == 0) {
+            double best = -1.0;
+            int bi = INT_MAX;
+            for (int i = jj + lane; i < m; i += 32) {
+                double v = cabs1(P[i + (int64_t)jj * ldp]);
+                if (v > best) {
+                    best = v;
+                    bi = i;
+                }
+            }
+#pragma unroll
+            for (int off = 16; off; off >>= 1) {
+                double ob = __shfl_xor_sync(FULL_MASK, best, off);
+                int oi = __shfl_xor_sync(FULL_MASK, bi, off);
+                if (ob > best || (ob == best && oi < bi)) {
+                    best = ob;
+                    bi = oi;
+                }
+            }
+            // IZAMAX starts from the first entry: a NaN there is returned as the pivot.
+            double first = cabs1(P[jj + (int64_t)jj * ldp]);
+            if (bi == INT_MAX || first != first) bi = jj;
+            double2 piv = P[bi + (int64_t)jj * ldp];
+            bool nz = (piv.x != 0.0 || piv.y != 0.0);
+            if (nz) {
+                if (bi != jj) {
+                    if (lane == 0) {
+                        P[bi + (int64_t)jj * ldp] = P[jj + (int64_t)jj * ldp];
+                        P[jj + (int64_t)jj * ldp] = piv;
+                    }
+                    if (Bs)
+                        for (int c = lane; c < nrhs; c += 32)
+                            swap2(Bs[jj + (int64_t)c * ldbs], Bs[bi + (int64_t)c * ldbs]);
+                }
+                __syncwarp();
+                double2 inv = crecip(piv);
+                for (int i = jj + 1 + lane; i < m; i += 32)
+                    P[i + (int64_t)jj * ldp] = cmul(P[i + (int64_t)jj * ldp], inv);
+            } else if (lane == 0 && *s_info == 0) {
+                *s_info = jj + 1;
+            }
+            if (lane == 0) {
+                s_bc[0] = bi;
+                s_bc[1] = nz ? 1 : 0;
+                ipiv[jj] = bi + 1;
+            }
+        }
+        __syncthreads();
+        const int p = s_bc[0];
+        const bool doswap = s_bc[1] && p != jj;
+        if (doswap)
+            for (int c = tid; c < jj; c += NT) swap2(P[jj + (int64_t)c * ldp], P[p + (int64_t)c * ldp]);
+        for (int c = jj + 1 + warp; c < ncols; c += NW) {
+            double2 *col = P + (int64_t)c * ldp;
+            if (doswap) {
+                if (lane == 0) swap2(col[jj], col[p]);
+                __syncwarp();
+            }
+            const double2 u = col[jj];
+            const double2 *lcol = P + (int64_t)jj * ldp;
+            for (int i = jj + 1 + lane; i < m; i += 32) col[i] = csubmul(col[i], lcol[i], u);
+        }
+        __syncthreads();
+    }
+}
 
 
 // One row of the blocked substitution: b[i, c] -= sum_j A[i, j] b[j, c] over the block's
@@ -289,6 +368,43 @@ __device__ void lu_solve_strips(const T *A, int64_t lda, int n, T *B, int ldb, i
     }
 }
 
+
+__global__ void __launch_bounds__(NT) sweep_fp64_smem_kernel(const RomDev *__restrict__ roms,
+                                                              const Item *__restrict__ items,
+                                                              int n_items, int *counter) {
+    extern __shared__ double2 smem[];
+    __shared__ int s_item, s_info, s_bc[2];
+    for (;;) {
+        const int it = next_item(counter, &s_item);
+        if (it >= n_items) break;
+        const Item w = items[it];
+        const RomDev R = roms[w.rom];
+        const int n = R.n;
+        const int lda = n | 1;
+        double2 *A = smem;
+        double2 *B = A + (int64_t)n * lda;
+        int *ipiv = reinterpret_cast<int *>(B + (int64_t)n * R.r);
+        assemble_into<double2>(A, lda, R, R.omega[w.f], w.f);
+        load_rhs(B, n, R);
+        if (threadIdx.x == 0) s_info = 0;
+        __syncthreads();
+        panel_factor_smem(A, lda, n, n, ipiv, &s_info, B, n, R.r, s_bc);
+        lu_solve<double2>(A, lda, n, B, n, R.r, nullptr);
+        store_solution(B, n, R, w.f);
+        if (R.LU) {
+            double2 *LU = R.LU + (int64_t)w.f * n * n;
+            for (int j = threadIdx.x >> 5; j < n; j += NW)
+                for (int i = threadIdx.x & 31; i < n; i += 32) LU[i + (int64_t)j * n] = A[i + j * lda];
+            for (int j = threadIdx.x; j < n; j += NT) R.ipiv[(int64_t)w.f * n + j] = ipiv[j];
+        }
+        if (threadIdx.x == 0) {
+            if (R.info) R.info[w.f] = s_info;
+            if (R.steps) R.steps[w.f] = 0;
+            if (R.berr) R.berr[w.f] = 0.0;
+        }
+        __syncthreads();
+    }
+}
 
 // ====================================================================================
 // global class
@@ -649,6 +765,38 @@ int64_t big_slot_bytes(int n_max) { return big_panel_offset(n_max) + (int64_t)(n
 size_t fp64_global_smem_bytes(int n_max, int r_max) { return global_smem_bytes(n_max, r_max, false); }
 
 int global_rpt(int n_max) { return (n_max + NT - 1) / NT; }
+
+// Where the shared-memory kernel is faster than the row kernel, by how the call's systems fill the GPU (a call alone,
+// row kernel / shared-memory kernel): a system a multiprocessor at most, order 1 and 1 right-hand side 30.7 / 24.1 us,
+// 8 and 16 43 / 35, 24 and 200 505 / 283, 1 and 5000 2135 / 350, but 16 and 1 36 / 41, 48 and 16 0.78 of the time; two a
+// multiprocessor (300 systems), order 4 and 32 right-hand sides 1.05, 8 and 64 0.94; four (600), order 2 and 64 1.04,
+// 3 and 64 0.94; more (1200, 4000), order 1 and 16 1.09 / 1.00, 2 and 64 1.08 / 0.95, 4 and 256 1.10 / 0.97.  Within a
+// first panel of 16 columns the row kernel has no second pass over the right-hand sides, hence the two lines.
+bool fp64_smem_faster(int n, int r, long long systems, int sms) {
+    const long long q = (long long)(n - 1) * (n - 1);
+    if (systems <= sms) return n <= 8 || (n <= 16 && 3LL * r >= n) || (n <= 32 && n > 16 && 5LL * r >= n);
+    if (n > 10) return false;
+    if (systems <= 2LL * sms + sms / 4) return r >= 2 * q;
+    if (systems <= 4LL * sms + sms / 4) return r >= 32 * q;
+    return r >= 16 + 26 * q;
+}
+
+cudaError_t launch_fp64_smem(const RomDev *roms, const Item *items, int n_items, int *counter,
+                             size_t smem, int grid, cudaStream_t st) {
+    auto k = sweep_fp64_smem_kernel;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<grid, NT, smem, st>>>(roms, items, n_items, counter);
+    return cudaGetLastError();
+}
+
+int fp64_smem_blocks_per_sm(size_t smem) {
+    int b = 0;
+    auto k = sweep_fp64_smem_kernel;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, NT, smem) != cudaSuccess) return 0;
+    return b;
+}
 
 // The mixed kernel takes all the shared memory a CTA may have (one CTA per SM either way, by
 // registers): what lies beyond its fixed regions deepens the correction solves' staging ring.

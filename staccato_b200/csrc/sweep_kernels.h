@@ -19,6 +19,12 @@ inline bool misaligned(const void *p, size_t a) { return p && (reinterpret_cast<
 // bytes of a whole n x n system with its right-hand sides and pivots: the small orders are those
 // whose system fits a CTA's shared memory
 size_t fp64_smem_bytes(int n, int r);
+// The shared-memory kernel (sweep.cu): the smallest orders and the widest right-hand sides; smem: the largest
+// system's bytes
+bool fp64_smem_faster(int n, int r, long long systems, int sms);
+int fp64_smem_blocks_per_sm(size_t smem);
+cudaError_t launch_fp64_smem(const RomDev *roms, const Item *items, int n_items, int *counter,
+                             size_t smem, int grid, cudaStream_t st);
 size_t fp64_global_smem_bytes(int n_max, int r_max);
 // dynamic shared memory of the global kernels; big: the large-order FP64 instances
 size_t global_smem_bytes(int n_max, int r_max, bool big = false);
