@@ -129,3 +129,20 @@ def test_small_orders_singular_and_nan(handle):
         a, b = rom.solutions(), X
         assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(a[~np.isnan(a)], b[~np.isnan(b)])
         assert np.array_equal(rom.info.cpu().numpy(), info)
+
+
+@pytest.mark.parametrize("specs", [
+    [(64, 1, 3), (65, 2, 1), (128, 1, 2), (129, 1, 1), (257, 1, 1)],   # one launch for all four thread counts
+    [(64, 1, 147), (65, 1, 1)], [(64, 1, 300), (100, 3, 290)], [(64, 1, 300), (100, 3, 293)],  # up to a wave of the larger, and past it
+    [(200, 1, 147), (300, 2, 1)], [(200, 1, 148), (300, 2, 1)],
+    [(40, 2, 1), (500, 1, 1)], [(33, 1, 200), (500, 1, 100)],
+])
+def test_row_classes_sharing_a_launch(handle, specs):
+    datas = [_data(n, r, F, seed=i) for i, (n, r, F) in enumerate(specs)]
+    roms = [_dev(d, keep=i == 0) for i, d in enumerate(datas)]
+    sweep(handle, roms)
+    for rom, d in zip(roms, datas):
+        _check(rom, d, ENDS)
+    ip = roms[0].ipiv.cpu().numpy().reshape(roms[0].F, -1)
+    K, M, D, eta, rhs, omega = datas[0]
+    assert np.array_equal(ip[0], O.zgetrf(O.assemble(K, M, D, eta, omega[0]))[1])
