@@ -360,7 +360,7 @@ SROM_API int srom_band_order(int64_t n_rows, int64_t nnz, const int64_t *rowptr,
  * through their own pool, or real-time loops in which cudaMalloc's implicit synchronisation
  * and possible failure are not acceptable.  It needs no handle; it runs on the current
  * device and the given stream (NULL = legacy default stream) and returns after enqueueing.
- * Scratch is a 33 MB array inside the library (descriptor, work list and 32 MiB of matrix
+ * Scratch is a 54 MB array inside the library (descriptor, work list and 51 MiB of matrix
  * slots), held on every device that loads the library until the process exits.
  * Limits: n <= 512, F <= 65536, and the blocked kernel's shared memory, about
  * 24 n r + 288 (n + 1) + 21 KB bytes, within the device's per-block limit (r <= 5 at n = 512,

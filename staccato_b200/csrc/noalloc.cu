@@ -26,16 +26,28 @@ constexpr int NOALLOC_MAX_N = 512;
 constexpr int NOALLOC_MAX_F = 65536;
 constexpr size_t NOALLOC_HDR_BYTES = 512;  // RomDev at 0, work counter at 256
 constexpr size_t NOALLOC_ITEM_BYTES = sizeof(srom::Item) * (size_t)NOALLOC_MAX_F;
-constexpr size_t NOALLOC_SLOT_BYTES = size_t(32) << 20;  // matrices of in-flight systems (7 at n = 512, r <= 5)
+constexpr size_t NOALLOC_SLOT_BYTES = size_t(51) << 20;  // matrices and right-hand sides of the systems in flight
 constexpr size_t NOALLOC_BYTES = NOALLOC_HDR_BYTES + NOALLOC_ITEM_BYTES + NOALLOC_SLOT_BYTES;
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
 static_assert(sizeof(srom::RomDev) <= 256, "descriptor must fit its header slot");
+// As many systems in flight as 32 MiB hold of n x n matrices alone, at most one a multiprocessor (8 at n = 512, 148 up to
+// n = 119), with the most right-hand sides that the entry point takes: with one system fewer, a call of exactly that
+// many takes a second wave (n = 512, 8 frequencies: 3.5 ms; 6.9 with 7 slots).
+constexpr bool noalloc_slots_suffice() {
+    for (int n = 33; n <= NOALLOC_MAX_N; ++n) {
+        const int r = (227 * 1024 - 288 * (n + 1) - 21 * 1024) / (24 * n);
+        const size_t flight = (size_t(32) << 20) / (16 * (size_t)n * n);
+        if ((flight < 148 ? flight : 148) * (size_t)srom::lu64_slot_bytes(n, r) > NOALLOC_SLOT_BYTES) return false;
+    }
+    return true;
+}
+static_assert(noalloc_slots_suffice(), "slots for the systems in flight");
 static_assert((NOALLOC_HDR_BYTES + NOALLOC_ITEM_BYTES) % 256 == 0, "slots must stay 256-byte aligned");
 
 }  // namespace
 
-// 33 MB: descriptor, work counter, work list (65536 frequencies) and 32 MiB of matrix slots.
+// 54 MB: descriptor, work counter, work list (65536 frequencies) and 51 MiB of slots.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
 namespace {

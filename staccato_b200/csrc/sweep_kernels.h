@@ -67,7 +67,11 @@ cudaError_t launch_global_big(const GlobalArgs &a, int grid, cudaStream_t st);
 // tensor cores; threads = 64, 128, 256 or 512, at least n_max ----
 constexpr int LU64_MAX_N = 512;
 int lu64_blocks_per_sm(int threads, int n_max);
-int64_t lu64_slot_bytes(int n_max, int r_max);  // global scratch per CTA
+constexpr int lu64_lda(int n) { return (n + 7) / 8 * 8; }
+// global scratch per CTA: the matrix and the right-hand sides
+constexpr int64_t lu64_slot_bytes(int n_max, int r_max) {
+    return ((int64_t)lu64_lda(n_max) * ((int64_t)n_max + r_max) * 16 + 127) / 128 * 128;
+}
 cudaError_t launch_lu64(int threads, const GlobalArgs &a, int grid, cudaStream_t st);
 
 // ---- FP64, large orders (sweep_large.cu): groups of systems advance panel by panel, several

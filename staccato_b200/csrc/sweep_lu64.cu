@@ -68,7 +68,7 @@ struct Cfg<512> {
 // touches then fall in different halves of the 32 banks.
 __host__ __device__ constexpr int ld4(int n) { return (n + 3) / 8 * 8 + 4; }
 // Leading dimension of the scratch matrix: columns start on 128-byte lines.
-__host__ __device__ constexpr int lda_of(int n) { return (n + 7) / 8 * 8; }
+__host__ __device__ constexpr int lda_of(int n) { return lu64_lda(n); }
 
 template <int NT_>
 struct Smem {
@@ -787,10 +787,6 @@ int lu64_blocks_per_sm(int threads, int n_max) {
         case 256: return blocks_per_sm<256>(n_max);
         default: return blocks_per_sm<512>(n_max);
     }
-}
-
-int64_t lu64_slot_bytes(int n_max, int r_max) {
-    return ((int64_t)lu64::lda_of(n_max) * ((int64_t)n_max + r_max) * 16 + 127) / 128 * 128;
 }
 
 cudaError_t launch_lu64(int threads, const GlobalArgs &a, int grid, cudaStream_t st) {
