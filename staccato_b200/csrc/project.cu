@@ -363,7 +363,7 @@ struct VtyWindow {
 
 // A warp's share is two 8-row bands by half of the tiles across: eight fragment reads for twelve MMAs (one
 // band by all tiles took thirteen, and the shared-memory datapath as long as the MMAs).  PAIRS: rows of even
-// length, copied 16 bytes at a time, a warp a row.
+// length, copied 16 bytes at a time.
 template <int TH, int MAXT, bool PAIRS>
 __global__ void __launch_bounds__(MAXT) vty_partial_kernel(int64_t N, VtyWindow w, int nm, int64_t chunks_per_cta,
                                                            double *__restrict__ partial) {
@@ -374,6 +374,11 @@ __global__ void __launch_bounds__(MAXT) vty_partial_kernel(int64_t N, VtyWindow 
     const int a_sz = 32 * lda, b_sz = 32 * ldb;
     const int stage = a_sz + nm * b_sz;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    // lanes to a row, and rows to a warp's pass, of the copies: a whole warp a row left most lanes of narrow windows
+    // idle (107,163 rows, one matrix: k = 8 0.140 ms, k = 16 0.140; with the lanes shared out 0.033 and 0.044)
+    constexpr int PER = PAIRS ? 2 : 1;
+    const int need = TH > 2 ? 32 : max(kap, kbp) / PER;  // TH > 2: more than 32 columns across
+    const int lpr = need <= 4 ? 4 : need <= 8 ? 8 : need <= 16 ? 16 : 32, rpw = 32 / lpr;
     const int mloc = warp / (2 * nbp), band0 = warp % (2 * nbp) / 2 * 2, t0 = (warp & 1) * th;
     const bool second = band0 + 1 < nband;
     const int nt = min(th, ntile - t0);
@@ -385,14 +390,13 @@ __global__ void __launch_bounds__(MAXT) vty_partial_kernel(int64_t N, VtyWindow 
         double *dst0 = sh + buf * stage;
         const int64_t r0 = ch * 32;
         const int nr = (int)min((int64_t)32, N - r0);
-        for (int row = warp; row < 32 * (1 + nm); row += nw) {
+        for (int row = warp * rpw + lane / lpr; row < 32 * (1 + nm); row += nw * rpw) {
             const int rr = row & 31, which = row >> 5;  // 0: Vt, else matrix which - 1
             const bool isa = which == 0;
             const int kk = isa ? w.ka : w.kb, kp = isa ? kap : kbp;
             double *dst = dst0 + (isa ? rr * lda : a_sz + (which - 1) * b_sz + rr * ldb);
             const double *src = isa ? w.Vt + (r0 + rr) * w.ldv : w.Y + (which - 1) * w.y_stride + (r0 + rr) * w.ldy;
-            constexpr int PER = PAIRS ? 2 : 1;
-            for (int c = PER * lane; c < kp; c += 32 * PER) {
+            for (int c = PER * (lane % lpr); c < kp; c += lpr * PER) {
                 const unsigned d = (unsigned)__cvta_generic_to_shared(dst + c);
                 if (rr < nr && c < kk) {
                     if constexpr (PAIRS) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + c));
