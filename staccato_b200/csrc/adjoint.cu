@@ -12,8 +12,8 @@
 // multiprocessor.  The terms: lambda^H U and W^T x of all frequencies and all rank terms are two
 // complex GEMMs, G x of all frequencies is one a dense parameter (zgemm.cu), and a warp a
 // (frequency, parameter) combines them; so U, W and G are read once a GEMM tile instead of once a
-// frequency.  Per-frequency contributions are summed in a fixed order: the gradient is
-// deterministic.
+// frequency.  Small calls, bound by launches, take their terms in the solve kernel (fused_terms).
+// Per-frequency contributions are summed in a fixed order: the gradient is deterministic.
 //
 // What bounds it: the solves read the kept factors once (F n^2 16 bytes from HBM) behind a chain of 2 n
 // dependent steps a frequency; 32-row blocks keep that chain at one warp's 32 steps a block with the
@@ -104,6 +104,63 @@ __device__ __forceinline__ void load_tile(const double2 *__restrict__ LU, int n,
         if (lane < bs) tile[c * ADJ_LDT + lane] = conj2(LU[(j0 + lane) + (int64_t)(j0 + c) * n]);
 }
 
+// coef(w) = c0 + c1 (i w) + c2 (-w^2); -Re(coef S)
+__device__ __forceinline__ double contribution(const DParamDev &P, double w, double2 S) {
+    const double2 coef = make_double2(P.c0.x - w * P.c1.y - w * w * P.c2.x, P.c0.y + w * P.c1.x - w * w * P.c2.y);
+    return -(coef.x * S.x - coef.y * S.y);
+}
+
+// All terms of one frequency by its CTA, from lambda and x (n x r each) in shared memory: a warp a rank term, a dense
+// matrix's columns shared out over the warps.  part: ADJ_NW entries a term.
+__device__ __forceinline__ void frequency_terms(const AdjointArgs &a, int f, double w, int n, int r, const double2 *lam,
+                                                const double2 *x, double2 *part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t = 0; t < a.n_terms; ++t) {
+        const DParamTerm T = a.terms[t];
+        const DParamDev &P = a.params[T.param];
+        const bool dense = P.kind != 0;
+        if (!dense && t % ADJ_NW != warp) continue;
+        double2 S = make_double2(0.0, 0.0);
+        if (dense) {
+            for (int i = lane; i < n; i += 32)
+                for (int c = 0; c < r; ++c) {
+                    double2 g = make_double2(0.0, 0.0);
+#pragma unroll 4
+                    for (int l = warp; l < n; l += ADJ_NW) g = cfma(P.G[i + (int64_t)l * n], x[l + c * n], g);
+                    S = cfma(conj2(lam[i + c * n]), g, S);
+                }
+            S = warp_sum2(S);
+        } else {
+            const double2 *u = P.U + (int64_t)T.k * n, *v = (P.W ? P.W : P.U) + (int64_t)T.k * n;
+            const double s = P.s ? P.s[T.k] : 1.0;
+            for (int c = 0; c < r; ++c) {
+                double2 p = make_double2(0.0, 0.0), q = p;
+                for (int i = lane; i < n; i += 32) {
+                    p = cfma(conj2(lam[i + c * n]), u[i], p);
+                    q = cfma(v[i], x[i + c * n], q);
+                }
+                p = warp_sum2(p);
+                q = warp_sum2(q);
+                S = cfma(make_double2(s * p.x, s * p.y), q, S);
+            }
+        }
+        if (lane == 0) part[t * ADJ_NW + (dense ? warp : 0)] = S;
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < a.n_params; j += ADJ_NT) {
+        const DParamDev &P = a.params[j];
+        double2 S = make_double2(0.0, 0.0);
+        for (int t = P.term0; t < P.term0 + P.nterm; ++t)
+            for (int q = 0; q < (P.kind != 0 ? ADJ_NW : 1); ++q) {
+                S.x += part[t * ADJ_NW + q].x;
+                S.y += part[t * ADJ_NW + q].y;
+            }
+        a.partial[(int64_t)f * a.n_params + j] = contribution(P, w, S);
+    }
+}
+
+// TERMS: the CTA takes its frequency's terms too (small calls; n r <= ADJ_B ADJ_LDT), and lambda may be null.
+template <bool TERMS>
 __global__ void __launch_bounds__(ADJ_NT, 4) adjoint_solve_kernel(AdjointArgs a) {
     extern __shared__ double2 sh[];
     __shared__ int s_item;
@@ -179,9 +236,20 @@ __global__ void __launch_bounds__(ADJ_NT, 4) adjoint_solve_kernel(AdjointArgs a)
             __syncthreads();
         }
         // lambda = P^T z
-        double2 *lam = a.lambda + (int64_t)f * n * r;
-        for (int c = warp; c < r; c += ADJ_NW)
-            for (int i = lane; i < n; i += 32) lam[perm[i] + (int64_t)c * n] = Y[i + (int64_t)c * n];
+        if (!TERMS || a.lambda) {
+            double2 *lam = a.lambda + (int64_t)f * n * r;
+            for (int c = warp; c < r; c += ADJ_NW)
+                for (int i = lane; i < n; i += 32) lam[perm[i] + (int64_t)c * n] = Y[i + (int64_t)c * n];
+        }
+        if constexpr (TERMS) {
+            double2 *part = dinv + ADJ_B + ADJ_B * ADJ_LDT + (n + 3) / 4;  // past perm
+            for (int c = warp; c < r; c += ADJ_NW)
+                for (int i = lane; i < n; i += 32) tile[perm[i] + c * n] = Y[i + c * n];
+            __syncthreads();
+            for (int e = tid; e < n * r; e += ADJ_NT) Y[e] = R.X[(int64_t)f * n * r + e];
+            __syncthreads();
+            frequency_terms(a, f, R.omega[f], n, r, tile, Y, part);
+        }
         __syncthreads();
     }
 }
@@ -199,12 +267,6 @@ __global__ void adjoint_pack_kernel(const DParamDev *__restrict__ params, const 
         Wa[i + (int64_t)t * n] = w[i];
     }
     if (threadIdx.x == 0) sa[t] = P.s ? P.s[T.k] : 1.0;
-}
-
-// coef(w) = c0 + c1 (i w) + c2 (-w^2); -Re(coef S)
-__device__ __forceinline__ double contribution(const DParamDev &P, double w, double2 S) {
-    const double2 coef = make_double2(P.c0.x - w * P.c1.y - w * w * P.c2.x, P.c0.y + w * P.c1.x - w * w * P.c2.y);
-    return -(coef.x * S.x - coef.y * S.y);
 }
 
 // One warp a (frequency, parameter) of the frequencies [f0, f0 + nf).  Low rank: S = sum over the
@@ -261,6 +323,16 @@ static size_t solve_smem_bytes(int n, int r) {
     return sizeof(double2) * ((size_t)n * r + ADJ_B + ADJ_B * ADJ_LDT) + sizeof(int) * (size_t)n;
 }
 
+// The solve kernel takes the terms too: calls of one wave (four CTAs a multiprocessor) whose terms are a few thousand
+// multiply-adds a thread at most.  Apart they are up to nine launches: n = 8, 64 frequencies, one rank term, two dense
+// 84 us apart, 42 together (48 with the one-launch kernel before the GEMMs); n = 24, three rank-8 and two dense 99 /
+// 56; n = 128, sixteen rank-8 180 / 142, 592 frequencies 221 / 182; but n = 200, r = 3, sixteen rank-8 and two dense
+// (3.9e5 multiply-adds) at 592 frequencies 547 / 596.
+static bool fused_terms(int n, int r, int n_terms, int n_dense, int F, int sms) {
+    const int64_t work = (int64_t)r * n * (2LL * (n_terms - n_dense) + (int64_t)n * n_dense);
+    return F <= 4 * sms && (int64_t)n * r <= ADJ_B * ADJ_LDT && n_terms <= 512 && work <= 1LL << 17;
+}
+
 static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
 // Frequencies a pass of the terms takes: its products (two a term and right-hand side, and n a
@@ -295,16 +367,27 @@ cudaError_t launch_adjoint(const AdjointArgs &a0, const DParamDev *params, const
     double2 *Sb = reinterpret_cast<double2 *>(take(sizeof(double2) * (size_t)fc * r * nt));
     double2 *GX = reinterpret_cast<double2 *>(w);
     bool lowrank = false;
-    for (int j = 0; j < a.n_params; ++j) lowrank = lowrank || (params[j].kind == 0 && params[j].nterm > 0);
+    int n_dense = 0;
+    for (int j = 0; j < a.n_params; ++j) {
+        lowrank = lowrank || (params[j].kind == 0 && params[j].nterm > 0);
+        n_dense += params[j].kind != 0 ? params[j].nterm : 0;
+    }
 
-    const size_t smem = solve_smem_bytes(n, r);
-    cudaError_t e = cudaFuncSetAttribute(adjoint_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const bool fused = fused_terms(n, r, nt, n_dense, F, sms);
+    if (fused) a.lambda = a0.lambda;
+    auto kernel = fused ? adjoint_solve_kernel<true> : adjoint_solve_kernel<false>;
+    const size_t smem = solve_smem_bytes(n, r) + (fused ? sizeof(double2) * (size_t)(1 + nt * ADJ_NW) : 0);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_solve_kernel, ADJ_NT, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, ADJ_NT, smem);
     if (e != cudaSuccess) return e;
-    adjoint_solve_kernel<<<std::min(F, sms * std::max(per_sm, 1)), ADJ_NT, smem, st>>>(a);
+    kernel<<<std::min(F, sms * std::max(per_sm, 1)), ADJ_NT, smem, st>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (fused) {
+        adjoint_reduce_kernel<<<a.n_params, 256, 0, st>>>(a.partial, F, a.n_params, dJdp);
+        return cudaGetLastError();
+    }
     // parameters without a term contribute nothing
     if ((e = cudaMemsetAsync(a.partial, 0, sizeof(double) * (size_t)F * a.n_params, st)) != cudaSuccess) return e;
     if (lowrank) {

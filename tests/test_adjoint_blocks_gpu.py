@@ -49,3 +49,40 @@ def test_backward_blocks(handle, n, r, F):
     for only in ([params[1]], [params[0]]):  # one kind alone
         j = params.index(only[0])
         assert abs(backward(handle, d, t(gb), only).item() - ref[j]) <= 1e-10 * max(np.abs(ref).max(), 1.0)
+
+
+# both sides of the rule that takes the terms into the solve kernel: one wave of frequencies, n r up to a tile, 512
+# terms, 2^17 multiply-adds a frequency; the lambda array must not matter
+@pytest.mark.parametrize("n,r,F,terms,dense", [(33, 32, 2, 5, 1), (33, 33, 2, 5, 1), (40, 1, 5, 512, 0), (40, 1, 5, 513, 0),
+                                               (128, 1, 3, 0, 8), (128, 1, 3, 1, 8), (128, 1, 600, 3, 1), (20, 2, 592, 3, 2),
+                                               (20, 2, 593, 3, 2), (3, 1, 1, 7, 3)])
+def test_backward_terms(handle, n, r, F, terms, dense):
+    import torch
+
+    rng = np.random.default_rng(100 * n + terms)
+    c = lambda s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    K, M = c((n, n)) + 2.0 * n ** 0.5 * np.eye(n), 0.1 * c((n, n))
+    rhs, omega, gb = c((n, r)), rng.uniform(0.2, 1.5, F), c((F, n, r))
+    d = DeviceRom.from_host(K, M, None, rhs, omega, keep_factors=True)
+    sweep(handle, [d], flags=_capi.SROM_FLAG_KEEP_FACTORS)
+    t = lambda a: torch.from_numpy(np.asarray(a)).cuda()
+    flat = lambda a: t(np.asfortranarray(a).ravel(order="F").astype(np.complex128))
+    U, W, s, G = c((n, max(terms, 1))), c((n, max(terms, 1))), rng.uniform(0.5, 2, max(terms, 1)), [c((n, n)) for _ in range(dense)]
+    first = min(terms, 2)
+    params = [Param(U=flat(U[:, :first]), W=flat(W[:, :first]), s=t(s[:first]), rank=first, c0=0.3 + 0.1j, c1=0.7, c2=-0.2j),
+              Param(U=flat(U[:, first:]), rank=terms - first, c2=1.0)] + [Param(G=flat(g), c0=1j, c1=0.5 - 0.5j) for g in G]
+    A = np.stack([K - w * w * M for w in omega])
+    X = np.linalg.solve(A, np.broadcast_to(rhs, (F, n, r)))
+    lam = np.linalg.solve(A.conj().transpose(0, 2, 1), gb)
+    mats = [(U[:, :first] * s[:first]) @ W[:, :first].T, U[:, first:terms] @ U[:, first:terms].T] + G
+    want, scale = [], []
+    for p, m in zip(params, mats):
+        coef = p.c0 + p.c1 * (1j * omega) + p.c2 * (-omega * omega)
+        S = np.einsum("fir,fir->f", lam.conj(), m @ X)
+        want.append(-(coef * S).real.sum())
+        scale.append((np.abs(coef) * np.linalg.norm(lam, axis=(1, 2)) * np.linalg.norm(X, axis=(1, 2))).sum() * np.linalg.norm(m))
+    g, lam_d = backward(handle, d, t(gb), params, want_lambda=True)
+    assert np.array_equal(g.cpu().numpy(), backward(handle, d, t(gb), params).cpu().numpy())
+    # the solves: 1e-10 as in the test above; the sums: n^2 terms an entry
+    assert np.abs(lam_d.cpu().numpy() - lam).max() <= 1e-10 * np.abs(lam).max()
+    assert (np.abs(g.cpu().numpy() - want) <= 1e-10 * np.maximum(np.array(scale), 1e-300)).all()
