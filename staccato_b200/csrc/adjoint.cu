@@ -97,6 +97,12 @@ __device__ __forceinline__ void block_products(const double2 *__restrict__ LU, i
     }
 }
 
+// The power of two that keeps a pivot's reciprocal in the normal range: y = v / u is (sc v) (1 / (sc u)).
+__device__ __forceinline__ double pivot_scale(double2 u) {
+    const double m = fmax(fabs(u.x), fabs(u.y));
+    return m < 0x1p-1000 ? 0x1p600 : m > 0x1p1000 ? 0x1p-600 : 1.0;
+}
+
 // The block's diagonal triangle, conjugated and transposed: tile[i * ADJ_LDT + j] = conj(LU[j0 + j, j0 + i])
 __device__ __forceinline__ void load_tile(const double2 *__restrict__ LU, int n, int j0, int bs, double2 *tile) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -163,7 +169,7 @@ __device__ __forceinline__ void frequency_terms(const AdjointArgs &a, int f, dou
 template <bool TERMS>
 __global__ void __launch_bounds__(ADJ_NT, 4) adjoint_solve_kernel(AdjointArgs a) {
     extern __shared__ double2 sh[];
-    __shared__ int s_item;
+    __shared__ int s_item, s_scaled;
     const RomDev R = *a.rom;
     const int n = R.n, r = R.r;
     double2 *Y = sh;                                          // n x r
@@ -187,20 +193,32 @@ __global__ void __launch_bounds__(ADJ_NT, 4) adjoint_solve_kernel(AdjointArgs a)
         for (int j0 = 0; j0 < n; j0 += ADJ_B) {
             const int bs = min(ADJ_B, n - j0);
             load_tile(LU, n, j0, bs, tile);
-            if (warp == ADJ_NW - 1 && lane < bs) dinv[lane] = crecip(conj2(LU[(j0 + lane) + (int64_t)(j0 + lane) * n]));
+            if (warp == ADJ_NW - 1) {
+                const double2 u = lane < bs ? conj2(LU[(j0 + lane) + (int64_t)(j0 + lane) * n]) : make_double2(1.0, 0.0);
+                const double sc = pivot_scale(u);
+                if (lane < bs) dinv[lane] = crecip(make_double2(u.x * sc, u.y * sc));
+                const bool scaled = __any_sync(FULL_MASK, sc != 1.0);
+                if (lane == 0) s_scaled = scaled;
+            }
             block_products(LU, n, j0, bs, 0, j0, Y, r);
             __syncthreads();
             for (int c = warp; c < r; c += ADJ_NW) {
                 double2 *y = Y + (int64_t)c * n + j0;
                 double2 v = lane < bs ? y[lane] : make_double2(0.0, 0.0);
                 const double2 di = lane < bs ? dinv[lane] : make_double2(0.0, 0.0);
-                for (int j = 0; j < bs; ++j) {
-                    // row j is complete in its lane; the others subtract conj(U[j, lane]) y_j
+                // row j is complete in its lane; the others subtract conj(U[j, lane]) y_j
+                auto step = [&](int j, double2 num) {
                     const double2 t = tile[min(lane, bs - 1) * ADJ_LDT + j];
-                    const double2 m = cfma(v, di, make_double2(0.0, 0.0));
+                    const double2 m = cfma(num, di, make_double2(0.0, 0.0));
                     const double2 yj = shfl2(m, j);
                     if (lane == j) v = m;
                     if (lane > j) v = cfma(make_double2(-t.x, -t.y), yj, v);
+                };
+                if (!s_scaled) {
+                    for (int j = 0; j < bs; ++j) step(j, v);
+                } else {
+                    const double sc = lane < bs ? pivot_scale(LU[(j0 + lane) + (int64_t)(j0 + lane) * n]) : 1.0;
+                    for (int j = 0; j < bs; ++j) step(j, make_double2(v.x * sc, v.y * sc));
                 }
                 if (lane < bs) y[lane] = v;
             }

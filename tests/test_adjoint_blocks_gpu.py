@@ -86,3 +86,29 @@ def test_backward_terms(handle, n, r, F, terms, dense):
     # the solves: 1e-10 as in the test above; the sums: n^2 terms an entry
     assert np.abs(lam_d.cpu().numpy() - lam).max() <= 1e-10 * np.abs(lam).max()
     assert (np.abs(g.cpu().numpy() - want) <= 1e-10 * np.maximum(np.array(scale), 1e-300)).all()
+
+
+@pytest.mark.parametrize("n,tiny", [(1, 1e-310), (3, 1e-310), (40, 3e-309), (2, 1e-305), (2, 1e305), (33, 1e306)])
+def test_backward_extreme_last_pivot(handle, n, tiny):
+    """A last pivot whose reciprocal is out of range (the forward solve divides by it): lambda divides too."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    k = rng.uniform(1.0, 2.0, n) * np.exp(1j * rng.uniform(0.0, 1.0, n))
+    k[-1] = tiny * (1.0 + 0.5j)
+    rhs = np.ones((n, 1)) + 0j
+    rhs[-1] = 3.0 * tiny
+    gb = np.ones((1, n, 1)) * (1.0 - 2.0j)
+    gb[0, -1] *= tiny
+    d = DeviceRom.from_host(np.diag(k), np.zeros((n, n)) + 0j, None, rhs, np.array([1.0]), keep_factors=True)
+    sweep(handle, [d], flags=_capi.SROM_FLAG_KEEP_FACTORS)
+    U = torch.from_numpy(np.ones(n) + 0j).cuda()
+    g, lam = backward(handle, d, torch.from_numpy(gb).cuda(), [Param(U=U, rank=1)], want_lambda=True)
+    # conj(k) as stored, scaled by a power of two into the normal range before the division
+    sc = 2.0 ** (-1000.0 * np.sign(np.log10(tiny)))
+    want = gb[0, :, 0] / k.conj()
+    want[-1] = (gb[0, -1, 0] * sc) / (k[-1].conj() * sc)
+    got = lam.cpu().numpy()[0, :, 0]
+    assert np.isfinite(got).all() and (np.abs(got - want) <= 8 * np.finfo(float).eps * np.abs(want)).all()
+    x = d.solutions()[0, :, 0]
+    assert abs(g.item() + (got.conj().sum() * x.sum()).real) <= 1e-13 * np.abs(got).sum() * np.abs(x).sum()
