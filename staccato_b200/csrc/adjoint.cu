@@ -395,7 +395,8 @@ cudaError_t launch_adjoint(const AdjointArgs &a0, const DParamDev *params, const
     if (fused) a.lambda = a0.lambda;
     auto kernel = fused ? adjoint_solve_kernel<true> : adjoint_solve_kernel<false>;
     const size_t smem = solve_smem_bytes(n, r) + (fused ? sizeof(double2) * (size_t)(1 + nt * ADJ_NW) : 0);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one value for all sizes: another thread's smaller launch must not lower it between this call and this launch
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, ADJ_NT, smem);

@@ -957,7 +957,8 @@ static cudaError_t vty_launch(int64_t N, const VtyWindow &w, int nm, int nblk, d
     const bool pairs = ((w.ldv | w.ldy | w.ka | w.kb) & 1) == 0 && (w.y_stride & 1) == 0 &&
                        ((reinterpret_cast<uintptr_t>(w.Vt) | reinterpret_cast<uintptr_t>(w.Y)) & 15) == 0;
     auto kf = pairs ? vty_partial_kernel<TH, MAXT, true> : vty_partial_kernel<TH, MAXT, false>;
-    cudaError_t e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one value for all sizes: another thread's smaller launch must not lower it between this call and this launch
+    cudaError_t e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     const int64_t n_chunks = (N + 31) / 32;
     const int64_t per = (n_chunks + nblk - 1) / nblk;

@@ -746,6 +746,10 @@ __global__ void __launch_bounds__(NT) sweep_global_kernel(GlobalArgs a) {
 // ====================================================================================
 // host-side launch helpers
 // ====================================================================================
+// What the kernels of this file are allowed to ask for, one value for all sizes: another thread's smaller launch of the
+// same kernel must not lower it between a launcher's call and its launch.
+constexpr size_t SMEM_DYN = SMEM_OPTIN - GLOBAL_STATIC_SMEM;
+
 size_t fp64_smem_bytes(int n, int r) {
     const size_t lda = (size_t)(n | 1);
     return sizeof(double2) * (lda * n + (size_t)n * r) + sizeof(int) * (size_t)n;
@@ -784,7 +788,7 @@ bool fp64_smem_faster(int n, int r, long long systems, int sms) {
 cudaError_t launch_fp64_smem(const RomDev *roms, const Item *items, int n_items, int *counter,
                              size_t smem, int grid, cudaStream_t st) {
     auto k = sweep_fp64_smem_kernel;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DYN);
     if (e != cudaSuccess) return e;
     k<<<grid, NT, smem, st>>>(roms, items, n_items, counter);
     return cudaGetLastError();
@@ -793,7 +797,7 @@ cudaError_t launch_fp64_smem(const RomDev *roms, const Item *items, int n_items,
 int fp64_smem_blocks_per_sm(size_t smem) {
     int b = 0;
     auto k = sweep_fp64_smem_kernel;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DYN) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, NT, smem) != cudaSuccess) return 0;
     return b;
 }
@@ -819,7 +823,7 @@ static cudaError_t launch_global_t(const GlobalArgs &a0, int grid, cudaStream_t 
         if (ring < 2 * (size_t)16 * a.n_max * sizeof(float2)) return cudaErrorInvalidValue;
     }
     a.smem_dyn = (int)smem;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem, SMEM_DYN));
     if (e != cudaSuccess) return e;
     k<<<grid, NT, smem, st>>>(a);
     return cudaGetLastError();

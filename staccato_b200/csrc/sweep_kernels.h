@@ -38,6 +38,7 @@ int64_t big_panel_offset(int n_max);
 int64_t big_slot_bytes(int n_max);
 constexpr int MIXED_MAX_R = 16;
 constexpr size_t GLOBAL_STATIC_SMEM = 4096;
+constexpr size_t SMEM_OPTIN = 227 * 1024;  // shared memory a CTA may have
 // Arguments of the global-storage kernels.
 struct GlobalArgs {
     const RomDev *roms;

@@ -610,7 +610,8 @@ template <int CS>
 static cudaError_t launch_panel(const Args &a, int systems, int j0, cudaStream_t st) {
     auto k = large_panel_kernel<CS>;
     const size_t smem = panel_smem(a.n_max);
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one value for all sizes: another thread's smaller launch must not lower it between this call and this launch
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_smem(LARGE_MAX_N));
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(CS, systems, 1);
@@ -633,11 +634,12 @@ int64_t large_slot_bytes(int n_max, int r_max) { return (int64_t)large::Slot(n_m
 
 cudaError_t launch_large(const LargeArgs &g, cudaStream_t st) {
     using namespace large;
-    if (g.n_max > LARGE_MAX_N || g.slot_bytes < large_slot_bytes(g.n_max, g.r_max)) return cudaErrorInvalidValue;
     const size_t bsm = back_smem(g.n_max, g.r_max);
+    if (g.n_max > LARGE_MAX_N || g.slot_bytes < large_slot_bytes(g.n_max, g.r_max) || bsm > SMEM_OPTIN)
+        return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(large_u12_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U12_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(large_schur_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCHUR_SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(large_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(large_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_OPTIN);
     if (e != cudaSuccess) return e;
     for (int i0 = 0; i0 < g.n_items; i0 += g.group) {
         const int ns = std::min(g.group, g.n_items - i0);

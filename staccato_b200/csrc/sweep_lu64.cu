@@ -766,7 +766,8 @@ template <int NT_>
 static cudaError_t launch(const GlobalArgs &a, int grid, cudaStream_t st) {
     auto k = sweep_lu64_kernel<NT_>;
     const size_t smem = Smem<NT_>(a.n_max).total;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one value for all sizes: another thread's smaller launch must not lower it between this call and this launch
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Smem<NT_>(NT_).total);
     if (e != cudaSuccess) return e;
     k<<<grid, NT_, smem, st>>>(a);
     return cudaGetLastError();

@@ -1105,7 +1105,8 @@ static cudaError_t launch_tc_t(const GlobalArgs &a0, int grid, cudaStream_t st) 
     GlobalArgs a = a0;
     const size_t smem = tc_smem_bytes(a.n_max, a.r_max);
     a.smem_dyn = (int)smem;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one value for all sizes: another thread's smaller launch must not lower it between this call and this launch
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(SMEM_OPTIN - GLOBAL_STATIC_SMEM));
     if (e != cudaSuccess) return e;
     k<<<grid, NT, smem, st>>>(a);
     return cudaGetLastError();
