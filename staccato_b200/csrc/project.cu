@@ -635,18 +635,17 @@ __global__ void __launch_bounds__(GS_CT) gs_chol_kernel(const double *__restrict
 #pragma unroll
         for (int q = 0; q < GS_CR; ++q) g[q] = fma(Cm[(int64_t)i * GS_B + a0 + 8 * q], hc, g[q]);
     }
+    bool tiny = false;
 #pragma unroll
     for (int q = 0; q < GS_CR; ++q) {
         const int a = a0 + 8 * q;
         // unit diagonal past a short panel
         g[q] = a < b && c < b ? Cm[(int64_t)(j0 + a) * GS_B + c] - g[q] : (a == c ? 1.0 : 0.0);
+        tiny = tiny || (a == c && g[q] < 0x1p-900);
         G[a][c] = g[q];
     }
-    __syncthreads();
     // G = L D L^T by rows: row j is final before step j, and R[j][c] = G[j][c] / sqrt(G[j][j])
-    for (int j = 0; j + 1 < b; ++j) {
-        // (columns of norm below about 1e-154: the reciprocal of their pivot overflows)
-        const double d = G[j][j], t = d < 0x1p-1000 ? G[j][c] / d : G[j][c] * __drcp_rn(d);
+    auto step = [&](int j, double t) {
 #pragma unroll
         for (int q = 0; q < GS_CR; ++q) {
             const int a = a0 + 8 * q;
@@ -656,6 +655,14 @@ __global__ void __launch_bounds__(GS_CT) gs_chol_kernel(const double *__restrict
             }
         }
         __syncthreads();
+    };
+    // columns of norm below about 1e-154 have pivots whose reciprocal overflows: panels with a small diagonal entry (a
+    // pivot is smaller by 2^-53 at most, short of breaking down) divide.  (Chosen pivot by pivot, the test cost every
+    // panel 1.5 us.)
+    if (__syncthreads_or(tiny)) {
+        for (int j = 0; j + 1 < b; ++j) step(j, G[j][c] / G[j][j]);
+    } else {
+        for (int j = 0; j + 1 < b; ++j) step(j, G[j][c] * __drcp_rn(G[j][j]));
     }
     if (a0 == 0) rd[c] = 1.0 / sqrt(G[c][c]);
     __syncthreads();
