@@ -552,10 +552,10 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
                        "n=%d with r=%d: the right-hand sides (n*r*16 bytes) exceed shared memory", P.b_nmax,
                        P.b_rmax);
     // FP64 systems of orders up to 512 run on the row kernel, with the thread count that srom_tune measured, if any,
-    // except where the shared-memory kernel is the faster one.  In a call of up to a system a multiprocessor the two
-    // launches add up: its small systems run in the shadow of the larger ones on the row kernel, or, where it is those
-    // with many right-hand sides to a column that end last, all of them on the shared-memory kernel, if they fit it
-    // (100 systems of order 24, r = 200 and one of order 100: 0.32 ms together, 0.22 + 0.28 apart).
+    // except where the shared-memory kernel is the faster one.  In a call of few systems the two launches add up: its
+    // small systems run in the shadow of the larger ones on the row kernel, or, where it is those with many right-hand
+    // sides to a column that end last, all of them on the shared-memory kernel, if they fit it (100 systems of order
+    // 24, r = 200 and one of order 100: 0.32 ms together, 0.22 + 0.28 apart).
     auto fp64_upto512 = [&](int i) {
         return cls[i] >= 0 && roms[i].n <= srom::LU64_MAX_N && (cls[i] == 0 || cls[i] == 2 || (cls[i] == 1 && !mixed));
     };
@@ -566,7 +566,7 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
         return fp64_upto512(i) && srom::fp64_smem_faster(roms[i].n, roms[i].r, fp64_systems, h->sm_count) &&
                srom::fp64_smem_bytes(roms[i].n, roms[i].r) + srom::GLOBAL_STATIC_SMEM <= (size_t)h->max_smem_optin;
     };
-    const bool one_wave = fp64_systems <= h->sm_count;
+    const bool one_wave = fp64_systems <= h->sm_count, few = fp64_systems <= 2LL * h->sm_count;
     bool row_needed = false, fit = true, tiny = true, wide = false;
     for (int i = 0; i < n_roms; ++i)
         if (fp64_upto512(i)) {
@@ -578,7 +578,7 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
     for (int i = 0; i < n_roms && one_wave && row_needed && fit; ++i)
         wide = wide || many_rhs(i) || (tiny && small(i) && roms[i].r >= roms[i].n);
     auto on_smem = [&](int i) {
-        return fp64_upto512(i) && (one_wave && row_needed ? wide || many_rhs(i) : small(i));
+        return fp64_upto512(i) && (few && row_needed ? wide || many_rhs(i) : small(i));
     };
     P.b_nmax = P.b_rmax = 0;
     for (int i = 0; i < n_roms; ++i) {

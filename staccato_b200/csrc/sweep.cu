@@ -771,14 +771,16 @@ size_t fp64_global_smem_bytes(int n_max, int r_max) { return global_smem_bytes(n
 int global_rpt(int n_max) { return (n_max + NT - 1) / NT; }
 
 // Where the shared-memory kernel is faster than the row kernel, by how the call's systems fill the GPU (a call alone,
-// row kernel / shared-memory kernel): a system a multiprocessor at most, order 1 and 1 right-hand side 30.7 / 24.1 us,
-// 8 and 16 43 / 35, 24 and 200 505 / 283, 1 and 5000 2135 / 350, but 16 and 1 36 / 41, 48 and 16 0.78 of the time; two a
-// multiprocessor (300 systems), order 4 and 32 right-hand sides 1.05, 8 and 64 0.94; four (600), order 2 and 64 1.04,
-// 3 and 64 0.94; more (1200, 4000), order 1 and 16 1.09 / 1.00, 2 and 64 1.08 / 0.95, 4 and 256 1.10 / 0.97.  Within a
-// first panel of 16 columns the row kernel has no second pass over the right-hand sides, hence the two lines.
+// row kernel / shared-memory kernel, us or their ratio): one wave of the latter, two CTAs a multiprocessor where its
+// shared memory holds two: order 1 and 1 right-hand side 30.7 / 24.1, 8 and 16 43 / 35, 24 and 200 505 / 283, 1 and 5000
+// 2135 / 350, 222 systems of order 5 33 / 30.5; but 16 and 1 36 / 41, 48 and 16 0.78.  Two a multiprocessor (300 systems):
+// order 4 and 32 right-hand sides 1.05, 8 and 64 0.94; four (600): order 2 and 64 1.04, 3 and 64 0.94; more (1200, 4000):
+// order 1 and 16 1.09 / 1.00, 2 and 64 1.08 / 0.95, 4 and 256 1.10 / 0.97.  Within a first panel of 16 columns the row
+// kernel has no second pass over the right-hand sides, hence the two lines up to order 32.
 bool fp64_smem_faster(int n, int r, long long systems, int sms) {
     const long long q = (long long)(n - 1) * (n - 1);
-    if (systems <= sms) return n <= 8 || (n <= 16 && 3LL * r >= n) || (n <= 32 && n > 16 && 5LL * r >= n);
+    const int wave = sms * (2 * (fp64_smem_bytes(n, r) + 1088) <= (size_t)228 * 1024 ? 2 : 1);
+    if (systems <= wave) return n <= 8 || (n <= 16 && 3LL * r >= n) || (n <= 32 && n > 16 && 5LL * r >= n);
     if (n > 10) return false;
     if (systems <= 2LL * sms + sms / 4) return r >= 2 * q;
     if (systems <= 4LL * sms + sms / 4) return r >= 32 * q;

@@ -56,7 +56,7 @@ def test_small_orders(handle, n, r):
     _check(rom, data)
 
 
-@pytest.mark.parametrize("n,r,load", [(1, 1, 1.0), (1, 1, 1.01), (8, 1, 1.0), (8, 1, 1.01), (3, 8, 2.0), (4, 18, 2.2), (4, 18, 2.3),
+@pytest.mark.parametrize("n,r,load", [(1, 1, 1.0), (1, 1, 1.01), (8, 1, 1.0), (8, 1, 1.01), (8, 1, 2.0), (8, 1, 2.01), (32, 300, 1.5), (24, 200, 1.5), (3, 8, 2.0), (4, 18, 2.2), (4, 18, 2.3),
                                       (2, 32, 4.0), (2, 32, 4.4), (1, 16, 5.0), (2, 64, 9.0)])
 def test_small_orders_by_fill(handle, n, r, load):
     data = _data(n, r, int(load * _sms()))
