@@ -57,6 +57,7 @@ struct srom_handle {
     srom::kry::PivotStats band_stats;
     // full pattern and RCM order of the last band factorisation, reused by a call on the same pattern
     srom::kry::PatternCache band_cache;
+    srom::kry::SideStream band_side;
     // per-launch profiling
     struct ProfRec {
         std::string name;
@@ -307,6 +308,7 @@ int srom_destroy(srom_handle *h) {
     if (h->d_zero) cudaFree(h->d_zero);
     if (h->d_zwork) cudaFree(h->d_zwork);
     h->band_cache.release();
+    h->band_side.release();
     if (h->h_meta) cudaFreeHost(h->h_meta);
     if (h->h_flag) cudaFreeHost(h->h_flag);
     if (h->meta_done) cudaEventDestroy(h->meta_done);
@@ -1288,6 +1290,7 @@ int srom_krylov_basis(srom_handle *h, int64_t n_rows, int64_t nnz, const int64_t
     h->band_stats = srom::kry::PivotStats{};
     a.stats = &h->band_stats;
     a.cache = &h->band_cache;
+    a.side = &h->band_side;
     h->band_cache.last_reused = false;
     std::string msg;
     ProfScope ps(h, "krylov_basis", n_points, 0.0, 0.0);
@@ -1336,6 +1339,7 @@ int srom_fom_sweep(srom_handle *h, int64_t n_rows, int64_t nnz, const int64_t *r
     h->band_stats = srom::kry::PivotStats{};
     a.stats = &h->band_stats;
     a.cache = &h->band_cache;
+    a.side = &h->band_side;
     h->band_cache.last_reused = false;
     std::string msg;
     ProfScope ps(h, "fom_sweep", n_freq, 0.0, 0.0);

@@ -1200,6 +1200,26 @@ void PatternCache::release() {
     last_reused = false;
 }
 
+cudaError_t SideStream::create() {
+    cudaError_t e = cudaSuccess;
+    if (!st) {
+        int lo = 0, hi = 0;
+        e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, hi);
+    }
+    if (e == cudaSuccess && !panel) e = cudaEventCreateWithFlags(&panel, cudaEventDisableTiming);
+    if (e == cudaSuccess && !rest) e = cudaEventCreateWithFlags(&rest, cudaEventDisableTiming);
+    return e;
+}
+
+void SideStream::release() {
+    if (st) cudaStreamDestroy(st);
+    if (panel) cudaEventDestroy(panel);
+    if (rest) cudaEventDestroy(rest);
+    st = nullptr;
+    panel = rest = nullptr;
+}
+
 namespace {
 
 // 64-bit hash of a CSR pattern (rowptr words, then colind in pairs): a multiply-xorshift step per
@@ -1238,18 +1258,13 @@ struct BandContext {
     BandContext(const BandContext &) = delete;
     BandContext &operator=(const BandContext &) = delete;
     ~BandContext() {  // before the buffers go: the side stream uses them too
-        if (F.side) {
-            cudaStreamSynchronize(F.side);
-            cudaStreamDestroy(F.side);
-        }
-        if (F.ev_panel) cudaEventDestroy(F.ev_panel);
-        if (F.ev_rest) cudaEventDestroy(F.ev_rest);
+        if (F.side) cudaStreamSynchronize(F.side);
     }
 
     // The pattern's full symmetric form and RCM order: from the handle's cache when it holds
     // this pattern, else computed on the host and uploaded (into the cache when there is one).
     int init(cudaStream_t stream, int64_t n_rows, int64_t nnz, const int64_t *rowptr, const int *colind, int base,
-             int upper, PatternCache *cache, Err &E) {
+             int upper, PatternCache *cache, SideStream *side, Err &E) {
         st = stream;
         n = n_rows;
         B.st = st;
@@ -1344,11 +1359,10 @@ struct BandContext {
         KCU(cudaFuncSetAttribute(solve_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)backward_smem(SOLVE_RMAX)));
         KCU(cudaMemsetAsync(F.d_ticket, 0, sizeof(unsigned), st));
-        int lo = 0, hi = 0;
-        KCU(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-        KCU(cudaStreamCreateWithPriority(&F.side, cudaStreamNonBlocking, hi));
-        KCU(cudaEventCreateWithFlags(&F.ev_panel, cudaEventDisableTiming));
-        KCU(cudaEventCreateWithFlags(&F.ev_rest, cudaEventDisableTiming));
+        KCU(side->create());
+        F.side = side->st;
+        F.ev_panel = side->panel;
+        F.ev_rest = side->rest;
         KCU(cudaFuncSetAttribute(ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(smem + sizeof(double2) * NB)));
         KCU(cudaFuncSetAttribute(trsv_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1400,7 +1414,7 @@ int krylov_basis(const KrylovArgs &a, std::string *msg, int *n_cols, KrylovLog *
     if (log) log->blocks.clear();
     if (a.n_rows == 0 || a.n_in == 0 || a.n_points == 0) return SROM_OK;
     BandContext X;
-    if (X.init(a.stream, a.n_rows, a.nnz, a.rowptr, a.colind, a.base, a.upper, a.cache, E)) {
+    if (X.init(a.stream, a.n_rows, a.nnz, a.rowptr, a.colind, a.base, a.upper, a.cache, a.side, E)) {
         *msg = E.msg;
         return E.code;
     }
@@ -1469,7 +1483,7 @@ int fom_sweep(const FomArgs &a, std::string *msg) {
     Err E;
     if (a.n_rows == 0 || a.r == 0 || a.n_freq == 0) return SROM_OK;
     BandContext X;
-    if (X.init(a.stream, a.n_rows, a.nnz, a.rowptr, a.colind, a.base, a.upper, a.cache, E)) {
+    if (X.init(a.stream, a.n_rows, a.nnz, a.rowptr, a.colind, a.base, a.upper, a.cache, a.side, E)) {
         *msg = E.msg;
         return E.code;
     }
