@@ -169,27 +169,21 @@ __device__ __forceinline__ bool same_columns(int64_t r0, const int64_t *__restri
 // arithmetic's time, and with fewer than 96 columns part of the lanes idle.  The gathers of 16 entries are in
 // flight together with the next 32 entries' columns and values.  An MMA adds its four products in order, so
 // the sums keep the order of the entries (Y's bits are those of spmm_rows); nodes whose rows differ in pattern
-// go through spmm_rows.  k and the row strides are even.  Bound by the gathers (a quarter-warp's 16-byte loads
+// go through spmm_rows.  k (at most 16 TP) and the row strides are even.  Bound by the gathers (a quarter-warp's 16-byte loads
 // fall in four lines).  Tet10 block: 0.20 -> 0.14 ms at k = 32, 0.22 -> 0.20 ms at k = 48.  One or three
 // matrices would fill three or nine rows of the eight: spmm_full_kernel.
 template <int TP>
 __global__ void __launch_bounds__(SPMM_THREADS, SPMM_MMA_CTAS) spmm_mma_kernel(int64_t N, const int64_t *__restrict__ rowptr,
                                                                    const int *__restrict__ colind, int base,
-                                                                   ProjVals vals, const double *__restrict__ Vt0, int k,
-                                                                   int ldv, double *__restrict__ Y0, int ldy,
+                                                                   ProjVals vals, const double *__restrict__ Vt, int k,
+                                                                   int ldv, double *__restrict__ Y, int ldy,
                                                                    int64_t y_stride) {
     __shared__ SpmmStage stage[SPMM_WARPS];
     const int lane = threadIdx.x & 31, lr = lane >> 2, lk = lane & 3;
     SpmmStage &st = stage[threadIdx.x >> 5];
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int nwin = (k + 16 * TP - 1) / (16 * TP);
-    const int64_t nodes = (N + 2) / 3;
-    for (int64_t it = warp; it < nodes * nwin; it += nwarp) {
-        const int64_t r0 = it % nodes * 3;
-        const int w0 = (int)(it / nodes) * 16 * TP, kw = min(16 * TP, k - w0);
-        const double *Vt = Vt0 + w0;
-        double *Y = Y0 + w0;
+    for (int64_t r0 = warp * 3; r0 < N; r0 += nwarp * 3) {
         const int nr = (int)min((int64_t)3, N - r0);
         const int64_t p0 = rowptr[r0], p1 = rowptr[r0 + 1], p2 = rowptr[min(r0 + 2, N)], p3 = rowptr[min(r0 + 3, N)];
         bool same = nr == 3 && p2 - p1 == p1 - p0 && p3 - p2 == p1 - p0;
@@ -233,7 +227,7 @@ __global__ void __launch_bounds__(SPMM_THREADS, SPMM_MMA_CTAS) spmm_mma_kernel(i
                         const bool live = c0 + 4 * (h + g) + lk < len;
 #pragma unroll
                         for (int u = 0; u < TP; ++u)
-                            v[g][u] = live && 16 * u + 2 * lr < kw ? *reinterpret_cast<const double2 *>(vr + 16 * u)
+                            v[g][u] = live && 16 * u + 2 * lr < k ? *reinterpret_cast<const double2 *>(vr + 16 * u)
                                                                    : make_double2(0.0, 0.0);
                     }
 #pragma unroll
@@ -252,14 +246,14 @@ __global__ void __launch_bounds__(SPMM_THREADS, SPMM_MMA_CTAS) spmm_mma_kernel(i
 #pragma unroll
                 for (int u = 0; u < TP; ++u) {
                     const int c = 16 * u + 4 * lk;
-                    if (c < kw) *reinterpret_cast<double2 *>(y + 16 * u) = make_double2(acc[u][0][0], acc[u][1][0]);
-                    if (c + 2 < kw) *reinterpret_cast<double2 *>(y + 16 * u + 2) = make_double2(acc[u][0][1], acc[u][1][1]);
+                    if (c < k) *reinterpret_cast<double2 *>(y + 16 * u) = make_double2(acc[u][0][0], acc[u][1][0]);
+                    if (c + 2 < k) *reinterpret_cast<double2 *>(y + 16 * u + 2) = make_double2(acc[u][0][1], acc[u][1][1]);
                 }
             }
         }
         if (!same)
             for (int r = 0; r < nr; ++r)
-                spmm_rows<(TP + 1) / 2, 2, 1>(r0 + r, rowptr, colind, base, vals, Vt, kw, ldv, Y, ldy, y_stride, lane, st);
+                spmm_rows<(TP + 1) / 2, 2, 1>(r0 + r, rowptr, colind, base, vals, Vt, k, ldv, Y, ldy, y_stride, lane, st);
     }
 }
 
