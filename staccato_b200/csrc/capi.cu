@@ -594,7 +594,9 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
             P.flops[0] += lu_flops(d.n, d.r) * d.F;
             continue;
         }
-        if (fp64_upto512(i)) cls[i] = CLS_ROW + row_class(d.n, tuned_wide(h, d.n, d.r));
+        // (the tuned thread count only in the FP64 form: measured at two systems a multiprocessor, it made the mixed
+        // forms' batches, where such orders are a small part of many systems, 0.3 % slower)
+        if (fp64_upto512(i)) cls[i] = CLS_ROW + row_class(d.n, !mixed && tuned_wide(h, d.n, d.r));
         const int c = cls[i];
         int *nm = c == 1 ? &P.g_nmax : c == 2 ? &P.b_nmax : c == 3 ? &P.t_nmax : &P.r_nmax[c - CLS_ROW];
         int *rm = c == 1 ? &P.g_rmax : c == 2 ? &P.b_rmax : c == 3 ? &P.t_rmax : &P.r_rmax[c - CLS_ROW];
