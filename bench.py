@@ -118,29 +118,21 @@ class ClockSampler:
 
 # ----------------------------------------------------------------------------- peaks
 
-# DRAM bytes (read + write) per launch of the dominant kernel of a form on this bench's default
-# workload (the 64-ROM batching draw of rank 0), keyed by (form, kernel).  The CUDA-core and FP64
-# global kernels: a one-pass ncu capture of dram__bytes_read.sum + dram__bytes_write.sum over
-# `bench.py --steps 1 --warmup 3 --no-cpu-baseline --no-e2e --no-extras` (mean of 4 launches;
-# the CUDA-core kernel then took every system of the mixed form, as it does in mixed_fp32).
-MEASURED_TRAFFIC = {("mixed_fp32", "mixed_global"): 574.5e9 + 460.1e9, ("fp64", "fp64_global"): 1757.4e9 + 1803.5e9}
-TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per launch, one-pass capture of this "
-                  "workload; compare with the bytes the matrices alone need (8 n^2 B per FP32 system, "
-                  "16 n^2 B per FP64 system)")
-# The tensor-core kernel of the headline (SROM_MIXED_AUTO) sweep: the same metrics captured on a
-# small case, every 16th frequency of every ROM of the same batch (same n / r mix, autotuned the
-# same way; one launch of 5,271 systems and 0.717 TFLOP), scaled to a full launch by its flops.
-TC_SAMPLE_BYTES = 42724239616 + 42177227776
-TC_SAMPLE_FLOPS = 716926045381.0
-TC_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the tensor-core launch on every 16th "
-                     "frequency of the same batch (84.9 GB for 0.717 TFLOP), scaled to this launch by its flops; "
-                     "compare with 8 n^2 B per FP32 system")
+# DRAM bytes (read + write) and algorithmic flops of a form's dominant kernels, captured by ncu
+# (dram__bytes_read.sum + dram__bytes_write.sum) on a small case of this bench's default workload: every
+# 16th frequency of every ROM of rank 0's batch (same n / r mix), scaled to a launch by its flops.
+TRAFFIC_SAMPLE = {"fp64_global": (98.556e9 + 104.223e9, 799.933e9),   # FP64 row kernel, 256 and 512 threads
+                  "mixed_global": (37.800e9 + 29.889e9, 803.573e9),   # CUDA-core mixed kernel
+                  "mixed_tc": (41.630e9 + 38.662e9, 659.724e9)}       # tensor-core mixed kernel
+TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the kernel's launches on every 16th frequency of "
+                  "the same batch, scaled to this launch by its flops; compare with the bytes the matrices alone need "
+                  "(8 n^2 B per FP32 system, 16 n^2 B per FP64 system)")
 
 
 # DRAM bytes (read + write) of one projection of the Tet10 block (K and M, k = 96): transpose,
 # SpMM, V^T Y and the partial reduction, from a one-pass ncu capture (dram__bytes_read.sum +
-# dram__bytes_write.sum) of the third projection of three; filled in from the capture.
-PROJ_TRAFFIC = 784.7e6
+# dram__bytes_write.sum) of the third projection of three.
+PROJ_TRAFFIC = 773.2e6
 PROJ_TRAFFIC_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum summed over the launches of one projection"
 
 
@@ -527,7 +519,7 @@ def krylov_leg(torch, dev, h):
     csr = DeviceCsr.from_host(K.indptr, K.indices, device=dev)
     Kd, Md, Dd, Bd = c(K.data), c(M.data), c(1e-5 * K.data + 2.0 * M.data), c(B.T)
     out = {"workload": "Tet10 block 10x10x40, N=%d, nnz=%d, 4 inputs" % (n, K.nnz), "bandwidth": bw,
-           "band_gb": band_b / 1e9, "solver": "band LDL^T (RCM order), trailing and solve updates on the library's complex FP64 tensor-core GEMM"}
+           "band_gb": band_b / 1e9, "solver": "band LDL^T (RCM order), trailing update on the FP64 tensor cores with look-ahead, one launch a block step in the solves"}
     for name, pts, order in (("one_point_order1", [100.0], 1), ("two_points_order4", [100.0, 800.0], 4)):
         torch.cuda.synchronize(dev)
         t0 = time.perf_counter()
@@ -658,7 +650,8 @@ def run_ours(args):
     h.set_stream(stream.cuda_stream)
     drom = [DeviceRom.from_host(r.K, r.M, r.D, r.rhs, r.omega, device=dev) for r in roms]
     # the autotuned schedule: srom_tune measures the kernel choices of every (n, r) of the batch
-    # (FP64 smem vs global kernel; the mixed form's FP64-outright vs mixed-kernel routing)
+    # (threads a system of the FP64 row kernel; the mixed form's FP64-outright vs mixed-kernel routing;
+    # CUDA-core vs tensor-core mixed kernel)
     t_tune = time.time()
     for rr in sorted({r.r for r in roms}):
         tune(h, sorted({r.n for r in roms if r.r == rr}), r=rr)
@@ -736,12 +729,11 @@ def run_ours(args):
         kms, kitems, kfl, kl = per[dom]
         achieved = kfl / (kms * 1e-3) / 1e12
         tot = sum(x[0] for x in per.values())
-        traffic, tsource = MEASURED_TRAFFIC.get((form, dom)), TRAFFIC_SOURCE
-        if form == "mixed" and dom == "mixed_tc" and kl > 0:
-            traffic, tsource = TC_SAMPLE_BYTES * (kfl / kl) / TC_SAMPLE_FLOPS, TC_TRAFFIC_SOURCE
+        sample = TRAFFIC_SAMPLE.get(dom)
+        traffic = sample[0] * (kfl / kl) / sample[1] if sample and kl > 0 else None
         return {"bound": "tensor", "achieved": achieved, "peak": peak,
                 "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic,
-                "traffic_source": tsource, "kernel": dom,
+                "traffic_source": TRAFFIC_SOURCE, "kernel": dom,
                 "peak_source": peak_source,
                 "algorithmic": "8/3 n^3 + 8 n^2 r real flops per system (LU + solve, both forms)",
                 "kernels": {k: {"ms_per_launch": v[0] / v[3], "launches": v[3],
@@ -879,11 +871,11 @@ def run_ours(args):
             "data": "synthetic",
             "config": {"workload": WORKLOAD, "systems_per_gpu": systems,
                        "tflop_per_step_per_gpu": flops / 1e12, "precision": headline,
-                       "refine": "complex-FP32 LU, each system on the faster of the two mixed kernels for its (n, r) as the autotuner measured (SROM_MIXED_AUTO: the tensor-core kernel, Schur updates as tcgen05 MMAs on three-piece bf16 splits, or the CUDA-core kernel; each measured on every system beside it as mixed_tc and mixed_fp32), FP64 residuals, <=5 corrections, each right-hand side stopping once its predicted error rho*||d||/||x|| (2-norms) <= 2^-34 (or the system early once the measured contraction cannot reach it), correction solves streamed through a shared-memory strip ring, back substitution by reciprocals of diag(U), FP64 fallback; systems the FP64 shared-memory kernel holds are routed by the autotuner (FP64 outright or a mixed kernel)",
+                       "refine": "complex-FP32 LU, each system on the faster of the two mixed kernels for its (n, r) as the autotuner measured (SROM_MIXED_AUTO: the tensor-core kernel, Schur updates as tcgen05 MMAs on three-piece bf16 splits, or the CUDA-core kernel; each measured on every system beside it as mixed_tc and mixed_fp32), FP64 residuals, <=5 corrections, each right-hand side stopping once its predicted error rho*||d||/||x|| (2-norms) <= 2^-34 (or the system early once the measured contraction cannot reach it), correction solves streamed through a shared-memory strip ring, back substitution by reciprocals of diag(U), FP64 fallback; systems that fit shared memory in FP64 (n <= ~112) are routed by the autotuner (FP64 outright or a mixed kernel), in SROM_MIXED_AUTO the other orders up to 320 are solved in FP64 outright (the call has more systems than multiprocessors)",
                        "l2": "inputs 167 MB + outputs 1.6 GB per step exceed L2; no flush",
-                       "autotune": "srom_tune over every (n, r) of the batch before warm-up (%.1f s): FP64 smem/global "
-                                   "kernel, the mixed form's FP64-outright/mixed-kernel routing of the orders the "
-                                   "FP64 smem kernel holds, and tensor-core vs CUDA-core mixed kernel for n in "
+                       "autotune": "srom_tune over every (n, r) of the batch before warm-up (%.1f s): threads a system of the "
+                                   "FP64 row kernel and the mixed form's FP64-outright/mixed-kernel routing of the "
+                                   "orders that fit shared memory, tensor-core vs CUDA-core mixed kernel for n in "
                                    "96..512" % tune_s,
                        "parallelism": f"independent batch per GPU x{world} (seed 3 + 1000003*rank)"},
             "roofline": info.get("roofline"),

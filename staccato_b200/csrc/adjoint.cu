@@ -20,7 +20,8 @@
 // products of the rows before it spread over all warps.  n = 128, 2000 frequencies, 16 rank-8
 // parameters and one dense (B200, the whole backward call): 2.4 ms with the dot products of every
 // row and every term taken by single warps, 0.40 ms now; the factors alone are 0.08 ms at the copy
-// bandwidth.
+// bandwidth.  Workspace beyond what the caller gives: the products of a pass (up to about 256 MB, kept in
+// the handle) and lambda (F n r) when it is not asked for.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -333,6 +334,8 @@ __global__ void __launch_bounds__(256) adjoint_reduce_kernel(const double *__res
     if (t == 0) out[j] = red[0];
 }
 
+// The limit that a call is refused by: two n x r blocks and an entry a term within a CTA's shared memory.  The kernels
+// above need less (solve_smem_bytes); the limit is part of the interface and stays.
 size_t adjoint_smem_bytes(int n, int r, int n_terms) {
     return sizeof(double2) * ((size_t)2 * n * r + (size_t)n_terms);
 }

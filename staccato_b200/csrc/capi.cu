@@ -546,6 +546,8 @@ int make_plan(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_
             P.b_nmax = std::max(P.b_nmax, roms[i].n);
             P.b_rmax = std::max(P.b_rmax, roms[i].r);
         }
+    // the limits of the interface (orders, and right-hand sides by the largest order beside the largest count, of the
+    // systems whose panel does not fit shared memory with them); the row kernel, which takes those up to 512, has none
     if (P.b_nmax > srom::BIG_MAX_N)
         return set_err(h, SROM_ERR_UNSUPPORTED, "n=%d exceeds the largest supported order %d", P.b_nmax,
                        srom::BIG_MAX_N);

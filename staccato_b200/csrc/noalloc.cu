@@ -136,7 +136,8 @@ extern "C" int srom_sweep_fp64_noalloc(const srom_rom_desc *d, void *cuda_stream
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
         return fail(err, err_len, SROM_ERR_CUDA, "cudaDeviceGetAttribute", cudaGetErrorString(e));
-    // the launch's own test (make_plan): rows per thread, and dynamic plus static shared memory
+    // the entry point's limit on n and r, that of a blocked kernel with its panel and right-hand sides in shared memory
+    // (the kernels below need less; slots are sized for it)
     if (srom::global_rpt(d->n) > srom::GLOBAL_MAX_RPT ||
         srom::fp64_global_smem_bytes(d->n, d->r) + srom::GLOBAL_STATIC_SMEM > (size_t)smem_optin) {
         char b[96];

@@ -7,11 +7,11 @@
 // basis comes from block Gram-Schmidt with re-orthogonalisation (KrylovROMSubstructure.cpp:433-454).
 //
 // B200 layout: V is transposed once into row-major Vt (N x k) so that the k entries of a
-// basis row are contiguous; the SpMM gives each warp one row and each lane k/32 basis
-// columns, and every gathered Vt row feeds all matrices of the pattern (K and M share it);
+// basis row are contiguous; the SpMM gives each warp one node (three rows), and every gathered
+// Vt row feeds its rows and all matrices of the pattern (K and M share it);
 // Y_m is written row-major.  R_m = Vt^T Y_m runs on the FP64 tensor cores
 // (mma.sync m8n8k4 f64): each CTA reduces a contiguous row range into a private k x k
-// partial, and a second kernel sums the partials in CTA order (deterministic).
+// partial, and a second kernel sums the partials in a fixed order (16 segments; deterministic).
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -170,7 +170,7 @@ __device__ __forceinline__ bool same_columns(int64_t r0, const int64_t *__restri
 // flight together with the next 32 entries' columns and values.  An MMA adds its four products in order, so
 // the sums keep the order of the entries (Y's bits are those of spmm_rows); nodes whose rows differ in pattern
 // go through spmm_rows.  k (at most 16 TP) and the row strides are even.  Bound by the gathers (a quarter-warp's 16-byte loads
-// fall in four lines).  Tet10 block: 0.20 -> 0.14 ms at k = 32, 0.22 -> 0.20 ms at k = 48.  One or three
+// fall in four lines).  Tet10 block: 0.20 -> 0.14 ms at k = 32, 0.22 -> 0.20 ms at k = 48 (TP = 3 spills 48 bytes).  One or three
 // matrices would fill three or nine rows of the eight: spmm_full_kernel.
 template <int TP>
 __global__ void __launch_bounds__(SPMM_THREADS, SPMM_MMA_CTAS) spmm_mma_kernel(int64_t N, const int64_t *__restrict__ rowptr,

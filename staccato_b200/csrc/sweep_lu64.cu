@@ -13,7 +13,7 @@
 //   2. U12     a chunk of trailing columns, a thread a column: the panel's interchanges, the unit
 //              triangle of the panel in 120 multiply-adds from registers, the result to the matrix
 //              and to shared memory as the MMA's B operand.
-//   3. Schur   32 x 16 warp tiles of the chunk's remaining rows, accumulators loaded from and
+//   3. Schur   16 x 16 warp tiles of the chunk's remaining rows, accumulators loaded from and
 //              stored to the matrix in the MMA's fragment layout.
 // With the right-hand sides as columns of the trailing matrix the forward substitution is part of
 // the factorisation, so L is neither written (unless the caller keeps the factors) nor read again;
@@ -27,13 +27,17 @@
 //     im: a' = (-a.y, -a.x) of k, k+1   b' = (b.x, b.y) of k, k+1.
 //
 // What bounds it: the chain of pivot steps (about 1300 cycles a column alone: reduction, reciprocal,
-// publishing the row, scaling) at orders up to about 200, with the FP64 pipe in the Schur updates above.
-// 128 registers a thread keep two (n <= 256), four (n <= 128) or six (n <= 64) systems an SM, so that
-// one system's pivot chain overlaps the others' Schur updates.
+// publishing the row, scaling) at orders up to about 200; above, the same chain and the Schur tiles that come from and
+// go to L2 (n = 512, 148 systems: issue slots 24 % busy, FP64 tensor pipe 33 %, L2 hit rate 50 %, stalls shared between
+// shared-memory and global loads and barriers).
+// Systems an SM, so that one's pivot chain overlaps the others' Schur updates: two up to n = 256 and four up to 128
+// by registers (128 a thread, 68 to 84 bytes of spills), five at n = 64 and six up to 60 by shared memory (168
+// registers a thread).
 // Measured on a B200, whole sweeps, against the kernels that it replaced (whole matrix in shared
 // memory, unblocked, up to n of about 112; 16-column panels with register-tiled fused multiply-adds,
 // one system an SM, above): n = 64, 500 systems, 318 -> 122 us; n = 189, 1000 systems, 4.9 -> 2.3 ms;
-// n = 256, r = 8, 2048 systems, 17.0 -> 9.3 ms.
+// n = 256, r = 8, 2048 systems, 17.0 -> 9.3 ms.  The whole-matrix kernel stays for the smallest orders and widest
+// right-hand sides (fp64_smem_faster in sweep.cu).
 #include <algorithm>
 #include <climits>
 
@@ -44,7 +48,7 @@ namespace lu64 {
 
 constexpr int NB = 16;  // panel width
 
-// blocks an SM by registers (128 a thread)
+// blocks an SM by registers; CW: columns of a chunk
 template <int NT_>
 struct Cfg;
 template <>
