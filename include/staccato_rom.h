@@ -140,12 +140,18 @@ SROM_API int srom_version(void);
  * test/krylovMidsizeTest/gpu/concurrent/batchedLU/src/main.cu:209-268 (which do not pivot).
  * All descriptor pointers are device pointers.  Asynchronous on the handle's stream.
  *
- * Sizes (B200, 227 KB of shared memory per block): the right-hand sides of a system live in
- * shared memory.  Orders whose 16-column panel also fits there (n <= 673 at r = 1, 548 at
- * r = 4, 314 at r = 16) run on the global kernel in every precision; larger ones, up to
- * n = 2560, on the large-order FP64 kernel, which needs n * r * 16 bytes + 64 KB (r <= 4 up to
- * n = 2559, r <= 8 up to n = 1388, r <= 16 up to n = 724); the mixed precisions solve those in
- * FP64 (steps = 0).  Requests beyond these limits return SROM_ERR_UNSUPPORTED.
+ * Sizes (B200, 227 KB of shared memory per block): the mixed kernels take the orders whose 16-column
+ * panel fits shared memory beside the right-hand sides (n <= 673 at r = 1, 548 at r = 4, 314 at
+ * r = 16); larger ones, up to n = 2560 and n * r * 16 bytes + 64 KB (r <= 4 up to n = 2559, r <= 8 up
+ * to n = 1388, r <= 16 up to n = 724), are solved in FP64 in every precision (steps = 0).
+ * Requests beyond these limits return SROM_ERR_UNSUPPORTED.
+ *
+ * Device memory of the handle (grows to the largest call, freed with the handle): a scratch slot
+ * a system in flight.  FP64, orders up to 512: (n rounded up to 8) x (n + r) x 16 bytes, 5 to 6 systems a
+ * multiprocessor up to n = 64 (49 MB in all at n = 64), 4 up to 128, 2 up to 256 (312 MB at n = 256), one up to
+ * 512 (622 MB); small orders that run whole in shared memory need none.  Larger orders: n x (n + r + 32) x 16
+ * bytes and at most one system a multiprocessor (15 GB for 148 frequencies of n = 2520).  Mixed
+ * forms: n x n x 16 bytes (tensor-core kernel: 2.7 MB at n = 512) and one a multiprocessor.
  */
 SROM_API int srom_sweep(srom_handle *h, const srom_rom_desc *roms, int n_roms, const srom_sweep_opts *opts);
 
